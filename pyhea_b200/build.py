@@ -7,6 +7,7 @@
 Run `python pyhea_b200/build.py` (or __graft_entry__.build()).  Objects are
 rebuilt when a source is newer than the library.
 """
+import concurrent.futures
 import glob
 import os
 import subprocess
@@ -20,6 +21,7 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 LIB = os.path.join(PKG, "libhea_cuda.so")
+OBJ = os.path.join(REPO, "build")  # object files
 EXT = os.path.join(PKG, "accelerate" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 
@@ -36,15 +38,21 @@ def _run(cmd):
 
 
 def build_lib(verbose_ptxas=False):
+    """One object per .cu file, compiled side by side, linked into the library."""
     cu = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
-    deps = cu + glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(INCLUDE, "*.h"))
-    if not _newer(LIB, deps) and not verbose_ptxas:
+    headers = (glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) +
+               glob.glob(os.path.join(INCLUDE, "*.h")))
+    if not _newer(LIB, cu + headers) and not verbose_ptxas:
         return LIB
-    cmd = [NVCC, *ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-shared", "-I", INCLUDE, "-I", CSRC,
-           "--expt-relaxed-constexpr", "-o", LIB, *cu]
-    if verbose_ptxas:
-        cmd[1:1] = ["-Xptxas", "-v"]
-    _run(cmd)
+    os.makedirs(OBJ, exist_ok=True)
+    flags = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I", INCLUDE, "-I", CSRC,
+             "--expt-relaxed-constexpr"] + (["-Xptxas", "-v"] if verbose_ptxas else [])
+    objects = [os.path.join(OBJ, os.path.basename(c)[:-3] + ".o") for c in cu]
+    jobs = [[NVCC, *ARCH, *flags, "-c", "-o", o, c] for c, o in zip(cu, objects)
+            if verbose_ptxas or _newer(o, [c] + headers)]
+    with concurrent.futures.ThreadPoolExecutor(max(1, os.cpu_count() or 1)) as pool:
+        list(pool.map(_run, jobs))
+    _run([NVCC, *ARCH, "-shared", "-o", LIB, *objects])
     return LIB
 
 

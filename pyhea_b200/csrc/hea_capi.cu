@@ -21,8 +21,8 @@
 #include <vector>
 
 #include "hea_cuda.h"
+#include "hea_kernels.h"
 #include "hea_search.cuh"
-#include "hea_large.cuh"
 
 using namespace hea;
 
@@ -154,75 +154,39 @@ void dev_free(void *p)
     } while (0)
 
 // ---------------------------------------------------------------------------
-// Kernel dispatch over (T, S)
+// Kernel dispatch: the instances of each species count live in a translation
+// unit of their own (hea_inst_t*.cu), found through its table.
 // ---------------------------------------------------------------------------
-using GenFn = void (*)(const SearchConst, const GenArgs);
-using McFn = void (*)(const SearchConst, const McArgs);
-
-#define HEA_GEN_ROW(T) {nullptr, generate_kernel<T, 1>, generate_kernel<T, 2>, generate_kernel<T, 3>}
-const GenFn kGen[kMaxTypes + 1][kMaxShells + 1] = {
-    {nullptr, nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr, nullptr}, HEA_GEN_ROW(2), HEA_GEN_ROW(3),
-    HEA_GEN_ROW(4), HEA_GEN_ROW(5), HEA_GEN_ROW(6)};
-
-// Local-search kernel for species count T and the table's padded shell layout:
-// the layouts of the FCC/BCC shell sets (in int4 chunks per shell) have their
-// loads unrolled; any other table uses the runtime-layout instance.
-template <int T>
-McFn pick_mc_t(int c0, int c1, int c2, int S, bool implicit)
-{
-    if (implicit) return S == 1 ? mc_kernel<T, ImplicitShells<1>> : S == 2 ? mc_kernel<T, ImplicitShells<2>>
-                                                                          : mc_kernel<T, ImplicitShells<3>>;
-    if (c0 == 2 && c1 == 0 && c2 == 0) return mc_kernel<T, Shells<2, 0, 0>>;  // BCC, 1 shell
-    if (c0 == 2 && c1 == 2 && c2 == 0) return mc_kernel<T, Shells<2, 2, 0>>;  // BCC, 2 shells
-    if (c0 == 2 && c1 == 2 && c2 == 3) return mc_kernel<T, Shells<2, 2, 3>>;  // BCC 8/6/12
-    if (c0 == 3 && c1 == 0 && c2 == 0) return mc_kernel<T, Shells<3, 0, 0>>;  // FCC, 1 shell
-    if (c0 == 3 && c1 == 2 && c2 == 0) return mc_kernel<T, Shells<3, 2, 0>>;  // FCC, 2 shells
-    if (c0 == 3 && c1 == 2 && c2 == 3) return mc_kernel<T, Shells<3, 2, 3>>;  // FCC 12/6/12
-    if (c0 == 3 && c1 == 2 && c2 == 6) return mc_kernel<T, Shells<3, 2, 6>>;  // FCC 12/6/24
-    if (S == 1) return mc_kernel<T, RuntimeShells<1>>;
-    if (S == 2) return mc_kernel<T, RuntimeShells<2>>;
-    return mc_kernel<T, RuntimeShells<3>>;
-}
-
-// The same choice for the HBM-occupancy (cluster) search.
-template <int T>
-McFn pick_mc_large_t(int c0, int c1, int c2, int S, bool implicit)
-{
-    if (implicit)
-        return S == 1 ? mc_large_kernel<T, ImplicitShells<1>>
-                      : S == 2 ? mc_large_kernel<T, ImplicitShells<2>> : mc_large_kernel<T, ImplicitShells<3>>;
-    if (c0 == 2 && c1 == 2 && c2 == 3) return mc_large_kernel<T, Shells<2, 2, 3>>;
-    if (c0 == 3 && c1 == 2 && c2 == 3) return mc_large_kernel<T, Shells<3, 2, 3>>;
-    if (c0 == 3 && c1 == 2 && c2 == 6) return mc_large_kernel<T, Shells<3, 2, 6>>;
-    if (S == 1) return mc_large_kernel<T, RuntimeShells<1>>;
-    if (S == 2) return mc_large_kernel<T, RuntimeShells<2>>;
-    return mc_large_kernel<T, RuntimeShells<3>>;
-}
-
-McFn pick_mc_large(int T, int c0, int c1, int c2, int S, bool implicit)
+const KernelSet &kernels(int T)
 {
     switch (T) {
-    case 2: return pick_mc_large_t<2>(c0, c1, c2, S, implicit);
-    case 3: return pick_mc_large_t<3>(c0, c1, c2, S, implicit);
-    case 4: return pick_mc_large_t<4>(c0, c1, c2, S, implicit);
-    case 5: return pick_mc_large_t<5>(c0, c1, c2, S, implicit);
-    default: return pick_mc_large_t<6>(c0, c1, c2, S, implicit);
+    case 2: return kernel_set_t2();
+    case 3: return kernel_set_t3();
+    case 4: return kernel_set_t4();
+    case 5: return kernel_set_t5();
+    default: return kernel_set_t6();
     }
 }
 
-using LGenFn = void (*)(const SearchConst, uint8_t *, const int32_t *, uint32_t);
-using LRecFn = void (*)(const SearchConst, const int4 *, const uint8_t *, const int32_t *, int32_t *, uint4 *);
-using LFitFn = void (*)(const SearchConst, const int32_t *, int, const int32_t *, double *);
-const LGenFn kLGen[kMaxTypes + 1] = {nullptr, nullptr, large_generate_kernel<2>, large_generate_kernel<3>,
-                                     large_generate_kernel<4>, large_generate_kernel<5>, large_generate_kernel<6>};
-#define HEA_LREC_ROW(T) {nullptr, large_recount_kernel<T, 1>, large_recount_kernel<T, 2>, large_recount_kernel<T, 3>}
-const LRecFn kLRec[kMaxTypes + 1][kMaxShells + 1] = {
-    {nullptr, nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr, nullptr}, HEA_LREC_ROW(2), HEA_LREC_ROW(3),
-    HEA_LREC_ROW(4), HEA_LREC_ROW(5), HEA_LREC_ROW(6)};
-#define HEA_LFIT_ROW(T) {nullptr, large_fitness_kernel<T, 1>, large_fitness_kernel<T, 2>, large_fitness_kernel<T, 3>}
-const LFitFn kLFit[kMaxTypes + 1][kMaxShells + 1] = {
-    {nullptr, nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr, nullptr}, HEA_LFIT_ROW(2), HEA_LFIT_ROW(3),
-    HEA_LFIT_ROW(4), HEA_LFIT_ROW(5), HEA_LFIT_ROW(6)};
+// ---------------------------------------------------------------------------
+// Stable ordering of populations by f2 (pyhea/cpp/accelerate.cpp:37-64,
+// :305-330): rank_i = #{j : f_j < f_i} + #{j < i : f_j == f_i}; order is
+// rewritten in rank order.  One CTA; `count` <= 2 * 65535.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(1024) sort_slots_kernel(int32_t *order, const double *f2, int count, int32_t *scratch)
+{
+    for (int i = threadIdx.x; i < count; i += blockDim.x) scratch[i] = order[i];
+    __syncthreads();
+    for (int i = threadIdx.x; i < count; i += blockDim.x) {
+        const double fi = f2[scratch[i]];
+        int r = 0;
+        for (int j = 0; j < count; ++j) {
+            const double fj = f2[scratch[j]];
+            r += (fj < fi) || (fj == fi && j < i);
+        }
+        order[r] = scratch[i];
+    }
+}
 
 __global__ void zero_counts_kernel(const int32_t *order, int count, int32_t *cnt, int ncount)
 {
@@ -230,17 +194,6 @@ __global__ void zero_counts_kernel(const int32_t *order, int count, int32_t *cnt
     if (p >= count) return;
     int32_t *g = cnt + (size_t)order[p] * ncount;
     for (int x = threadIdx.x; x < ncount; x += blockDim.x) g[x] = 0;
-}
-
-McFn pick_mc(int T, int c0, int c1, int c2, int S, bool implicit)
-{
-    switch (T) {
-    case 2: return pick_mc_t<2>(c0, c1, c2, S, implicit);
-    case 3: return pick_mc_t<3>(c0, c1, c2, S, implicit);
-    case 4: return pick_mc_t<4>(c0, c1, c2, S, implicit);
-    case 5: return pick_mc_t<5>(c0, c1, c2, S, implicit);
-    default: return pick_mc_t<6>(c0, c1, c2, S, implicit);
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -818,20 +771,21 @@ int build_tables(const hea_problem *pb, uint64_t seed, DeviceTables &dt, int32_t
     }
 
     // shared memory of the two kernels
+    const KernelSet &ks = kernels(T);
     const size_t cnt_bytes = 4 * (size_t)((dt.ncount + 3) & ~3);
     dt.smem_gen = (size_t)c.occ_stride + 16 + cnt_bytes;
     dt.smem_mc = mc_smem(c.occ_stride, T, S, 16);  // the largest block (512 threads)
     if (dt.smem_mc > (size_t)smem_limit() || (flags & HEA_FLAG_HBM_OCCUPANCY)) {
         // structures beyond shared memory: occupancy in HBM, cluster search
         dt.large = true;
-        dt.mc = pick_mc_large(T, c.chunks[0], S > 1 ? c.chunks[1] : 0, S > 2 ? c.chunks[2] : 0, S, c.lat.L > 0);
-        dt.lgen = kLGen[T];
-        dt.lrec = kLRec[T][S];
-        dt.lfit = kLFit[T][S];
+        dt.mc = ks.mc_large(c.chunks[0], S > 1 ? c.chunks[1] : 0, S > 2 ? c.chunks[2] : 0, S, c.lat.L > 0);
+        dt.lgen = ks.lgen;
+        dt.lrec = ks.lrec[S];
+        dt.lfit = ks.lfit[S];
         HEA_CUDA(allow_max_smem(dt.mc));
     } else {
-        dt.gen = kGen[T][S];
-        dt.mc = pick_mc(T, c.chunks[0], S > 1 ? c.chunks[1] : 0, S > 2 ? c.chunks[2] : 0, S, c.lat.L > 0);
+        dt.gen = ks.gen[S];
+        dt.mc = ks.mc(c.chunks[0], S > 1 ? c.chunks[1] : 0, S > 2 ? c.chunks[2] : 0, S, c.lat.L > 0);
         HEA_CUDA(allow_max_smem(dt.gen));
         HEA_CUDA(allow_max_smem(dt.mc));
     }
@@ -1796,7 +1750,7 @@ extern "C" int hea_recount_noalloc(const hea_problem *problem, int32_t count, co
     int32_t *d_order = reinterpret_cast<int32_t *>(sc + o_order);
     int *d_err = reinterpret_cast<int *>(sc + o_err);
 
-    const GenFn gen = kGen[T][S];
+    const GenFn gen = kernels(T).gen[S];
     HEA_CUDA(allow_max_smem(gen));
     HEA_CUDA(cudaMemcpy(d_raw, pb->nbor, raw_bytes, cudaMemcpyHostToDevice));
     HEA_CUDA(cudaMemset(d_err, 0, sizeof(int)));

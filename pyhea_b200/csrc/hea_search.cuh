@@ -1157,24 +1157,4 @@ __global__ void __launch_bounds__(512, HEA_MC_MIN_BLOCKS) mc_kernel(const Search
     }
 }
 
-// ---------------------------------------------------------------------------
-// Stable ordering of populations by f2 (pyhea/cpp/accelerate.cpp:37-64,
-// :305-330): rank_i = #{j : f_j < f_i} + #{j < i : f_j == f_i}; order is
-// rewritten in rank order.  One CTA; `count` <= 2 * 65535.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) sort_slots_kernel(int32_t *order, const double *f2, int count, int32_t *scratch)
-{
-    for (int i = threadIdx.x; i < count; i += blockDim.x) scratch[i] = order[i];
-    __syncthreads();
-    for (int i = threadIdx.x; i < count; i += blockDim.x) {
-        const double fi = f2[scratch[i]];
-        int r = 0;
-        for (int j = 0; j < count; ++j) {
-            const double fj = f2[scratch[j]];
-            r += (fj < fi) || (fj == fi && j < i);
-        }
-        order[r] = scratch[i];
-    }
-}
-
 }  // namespace hea

@@ -101,8 +101,9 @@ int hea_cuda_available(void);
 const char *hea_last_error(void);
 
 /* Device buffers of finished searches are cached for the next search of the
- * same shape (up to 8 GiB per process); this returns the current device's
- * cached buffers to the driver.  No counterpart in the reference. */
+ * same shape (up to 8 GiB per process), and their streams and events for the
+ * next plan; this returns the current device's cached buffers and streams to
+ * the driver.  No counterpart in the reference. */
 void hea_release_cached_memory(void);
 
 /* L2 read bandwidth of the current device, the denominator of the search

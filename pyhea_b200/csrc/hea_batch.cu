@@ -1,115 +1,7 @@
-// hea_batch.cuh -- the job engine: many independent structures searched by one
-// persistent kernel.  It serves both the batch API (hea_batch_*: a fixed set
-// of structures in one graph-captured launch) and the serving loop
-// (hea_server_*: structures admitted while others run, in time slices).
-//
-// Every structure runs the same search as the plain path (hea_search.cuh) with
-// its own constants, tables, population pools and Philox key, so its result
-// is bit-identical to searching it alone, whatever else shares the GPU.  Its
-// work is a sequence of phases of jobs:
-//
-//   phase 0        P x GEN0 (generation 0 of the population) and, when I > 0,
-//                  P x GENMC(0) (generation 1 of the new population, then its
-//                  local search, mc_call 0)
-//   phase k, 1..I  P x MC2(k-1) (local search of the survivors, mc_call
-//                  2(k-1)+1) and, when k < I, P x GENMC(k) (generation k+1,
-//                  local search with mc_call 2k)
-//
-// The CTA that finishes the last job of a structure's phase runs the phase
-// transition itself -- stable sort of the survivors, then the merge
-// (pyhea/cpp/accelerate.cpp:305-330, :693) -- and appends the next phase's
-// jobs.  With a tolerance, a local search also ends once its f2 is at or
-// below it, and the structure ends once the best f2 after a survivors' sort
-// is (the search of the population generated meanwhile is dropped).
-//
-// Jobs live in ring queues, one per priority level, whose head and tail only
-// grow; a CTA takes the next reserved job of the highest level that has one
-// and waits for the producer's sequence number in the slot.  A ring needs
-// room for the jobs of one phase of every structure at its level (at most
-// 2P each), since a phase is queued only after the previous one finished.
-//
-// A launch ends when no structure is active or, for the time slices of the
-// serving loop, at its deadline: CTAs stop taking jobs, and a local search
-// that sees the deadline stops at the end of its round, saves its state
-// (occupancy, counts, f2) to HBM and queues a continuation that resumes at
-// the next round with the same rejection count -- the same proposals follow,
-// so the result does not depend on where the slices fell.  Waits are bounded
-// by wall time since the last finished job; on expiry the kernel sets an
-// error flag and every CTA returns.
-//
-// Occupancy in HBM (`hbm`, the default: proposals are scored from the site
-// histograms, so a search reads the occupancy only for its draws): a job
-// converts the row to 5*species in place (reads through L2, so no stale L1
-// line of another SM's writes is used; the conversion rewrites every byte this
-// CTA later reads), searches it through L1, and converts it back.  Otherwise
-// the row is staged in the launch's shared memory.
-#pragma once
-#include <cstdint>
-
-#include "hea_search.cuh"
+// hea_batch.cu -- the job engine's kernels (hea_batch.h says how they work).
+#include "hea_batch.h"
 
 namespace hea {
-
-enum BatchJobKind : int32_t { kJobGen0 = 0, kJobGenMc = 1, kJobMc2 = 2 };
-
-struct BatchJob {
-    int32_t structure, kind, index, iter;
-    int32_t seq;     // low 32 bits of (ring position + 1), written after the other fields
-    int32_t resume;  // 1: continue a stopped local search at round0 with miss0 rejections
-    int32_t round0, miss0;
-};
-static_assert(sizeof(BatchJob) == 32, "BatchJob layout");
-
-// Kernel instance of a structure: species count and shell layout.
-enum BatchLayout : int32_t {
-    kLayBcc = 0, kLayFccTrue = 1, kLayRt1 = 2, kLayRt2 = 3, kLayRt3 = 4, kLayImp1 = 5, kLayImp2 = 6, kLayImp3 = 7
-};
-
-struct BatchStruct {
-    SearchConst c;
-    const int4 *nbor;
-    uint8_t *occ;
-    int32_t *cnt;
-    double *f2;
-    int32_t *order;    // [2P] slot ids
-    int32_t *scratch;  // [2P] sort scratch
-    uint4 *hist;       // [2P][N] site histograms
-    const uint32_t *nbmask;
-    int32_t P, Q, D, I;
-    int64_t max_rounds;
-    double tol2;  // tolerance on f2 (< 0: none): local searches and the structure end once reached
-    int32_t T, layout, level, hbm;
-};
-
-static_assert(sizeof(SearchConst) % 8 == 0 && alignof(SearchConst) >= 8, "SearchConst copied as 8-byte words");
-
-struct BatchState {
-    int32_t remaining;  // jobs of the current phase not finished
-    int32_t phase;      // at the end: the iterations run
-    int32_t done;       // 1 once the structure's search ended
-    int32_t pad_;
-    unsigned long long tally[3];  // rounds, evals, accepts of this structure
-};
-
-constexpr int kBatchLevels = 16;
-
-struct BatchQueue {
-    unsigned long long head;  // jobs taken
-    unsigned long long tail;  // jobs reserved by producers
-    unsigned long long cap;   // ring slots
-    unsigned long long base;  // first slot of this ring in the job array
-};
-
-struct BatchCtl {
-    BatchQueue q[kBatchLevels];
-    unsigned long long stats[4];  // rounds, evals, accepts, finished structures
-    int32_t error;                // 1: a wait ran out of time, 2: a ring slot was overwritten
-    int32_t active;               // structures seeded and not finished
-    unsigned long long wait_limit_ns;
-    unsigned long long start_ns;     // device time origin of finish times
-    unsigned long long deadline_ns;  // device time after which no job starts (0: none)
-    unsigned long long progress_ns;  // device time of the last finished job
-};
 
 // Stable ascending order of order[0, count) by f2 (rank counting); block-wide,
 // barriers inside.  scratch holds `count` ints.  Reads go through L2: the
@@ -323,13 +215,6 @@ __device__ __forceinline__ JobEnd batch_dispatch_t(const SearchConst &c, const B
     }
 }
 
-#ifndef HEA_BATCH_THREADS
-#define HEA_BATCH_THREADS 256
-#endif
-#ifndef HEA_BATCH_MIN_BLOCKS
-#define HEA_BATCH_MIN_BLOCKS 3  // resident CTAs per SM the register budget aims for (measured: 3 > 2, 4)
-#endif
-
 // The persistent kernel: CTAs take jobs until no structure is active or the
 // launch's deadline has passed.  Dynamic shared memory: occupancy of the
 // largest shared-memory structure + 16 + per-warp counts + swap records; the
@@ -449,5 +334,8 @@ __global__ void __launch_bounds__(HEA_BATCH_THREADS, HEA_BATCH_MIN_BLOCKS)
         if (k + 1 < I) enqueue_jobs(jobs, ctl, d.level, s, kJobGenMc, k + 1, P, &first);
     }
 }
+
+BatchFn batch_kernel_fn() { return batch_kernel; }
+BatchSeedFn batch_seed_kernel_fn() { return batch_seed_kernel; }
 
 }  // namespace hea

@@ -1,6 +1,7 @@
 // hea_capi.cu -- C ABI of the swap-search engine: validation, device tables,
 // the search driver and the component entry points.  Declarations and the
 // reference interfaces they replace: include/hea_cuda.h.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -147,6 +148,95 @@ void dev_free(void *p)
     P.cached += key.second;
 }
 
+// ---------------------------------------------------------------------------
+// Streams (each with two events) of finished plans, kept for the next plan in
+// the same context: a call that makes a plan of its own otherwise spends more
+// on creating and destroying them than on a small structure's kernels
+// (measured: a one-structure recount 395 -> 164 us; a 432-site search with
+// four populations ahead 1.31 -> 0.73 ms).
+// At most kQueuesKept stay; owners give a queue back once it is idle.
+// ---------------------------------------------------------------------------
+struct Queue {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t ev[2] = {nullptr, nullptr};
+    bool main = false;  // high priority and timing events (a plan's own stream); else low, without
+    CUcontext ctx = nullptr;
+};
+struct QueuePool {
+    std::mutex mu;
+    std::vector<Queue> kept;
+};
+QueuePool &queue_pool()
+{
+    static QueuePool *p = new QueuePool;  // never destroyed, like the block cache
+    return *p;
+}
+constexpr size_t kQueuesKept = 64;
+
+// The calling thread's context (streams belong to one); NULL where it cannot be told.
+CUcontext current_context()
+{
+    static CUresult (*const get)(CUcontext *) = [] {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &fn, cudaEnableDefault, &found) != cudaSuccess) {
+            cudaGetLastError();
+            fn = nullptr;
+        }
+        return reinterpret_cast<CUresult (*)(CUcontext *)>(fn);
+    }();
+    CUcontext ctx = nullptr;
+    if (!get || get(&ctx) != CUDA_SUCCESS) return nullptr;
+    return ctx;
+}
+
+void queue_destroy(const Queue &q)
+{
+    for (cudaEvent_t e : q.ev)
+        if (e) cudaEventDestroy(e);
+    if (q.stream) cudaStreamDestroy(q.stream);
+}
+
+int queue_take(bool main, Queue *out)
+{
+    HEA_CUDA(cudaFree(nullptr));  // the device's context is current from here on
+    const CUcontext ctx = current_context();
+    if (ctx) {
+        QueuePool &P = queue_pool();
+        std::lock_guard<std::mutex> lk(P.mu);
+        for (size_t i = P.kept.size(); i-- > 0;)
+            if (P.kept[i].ctx == ctx && P.kept[i].main == main) {
+                *out = P.kept[i];
+                P.kept.erase(P.kept.begin() + i);
+                return HEA_OK;
+            }
+    }
+    out->main = main;
+    out->ctx = ctx;
+    int least = 0, greatest = 0;
+    HEA_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    HEA_CUDA(cudaStreamCreateWithPriority(&out->stream, cudaStreamNonBlocking, main ? greatest : least));
+    for (cudaEvent_t &e : out->ev) HEA_CUDA(cudaEventCreateWithFlags(&e, main ? 0u : cudaEventDisableTiming));
+    return HEA_OK;
+}
+
+// Back to the pool; the queue's work has ended and ended well, else it is destroyed.
+void queue_give(Queue &q)
+{
+    if (!q.stream) {
+        queue_destroy(q);
+        return;
+    }
+    const bool idle = cudaStreamSynchronize(q.stream) == cudaSuccess;
+    QueuePool &P = queue_pool();
+    std::lock_guard<std::mutex> lk(P.mu);
+    if (idle && q.ctx && q.ev[0] && q.ev[1] && P.kept.size() < kQueuesKept)
+        P.kept.push_back(q);
+    else
+        queue_destroy(q);
+    q = Queue{};
+}
+
 #define HEA_TRY(expr)            \
     do {                         \
         int rc_ = (expr);        \
@@ -170,12 +260,15 @@ const KernelSet &kernels(int T)
 
 // ---------------------------------------------------------------------------
 // Stable ordering of populations by f2 (pyhea/cpp/accelerate.cpp:37-64,
-// :305-330): rank_i = #{j : f_j < f_i} + #{j < i : f_j == f_i}; order is
-// rewritten in rank order.  One CTA; `count` <= 2 * 65535.
+// :305-330): rank_i = #{j : f_j < f_i} + #{j < i : f_j == f_i} over the slots
+// of a[0, na) followed by b[0, nb); both are rewritten in rank order.  One CTA;
+// na + nb <= 2 * 65535.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) sort_slots_kernel(int32_t *order, const double *f2, int count, int32_t *scratch)
+__global__ void __launch_bounds__(1024) sort_slots_kernel(int32_t *a, int na, int32_t *b, int nb, const double *f2,
+                                                          int32_t *scratch)
 {
-    for (int i = threadIdx.x; i < count; i += blockDim.x) scratch[i] = order[i];
+    const int count = na + nb;
+    for (int i = threadIdx.x; i < count; i += blockDim.x) scratch[i] = i < na ? a[i] : b[i - na];
     __syncthreads();
     for (int i = threadIdx.x; i < count; i += blockDim.x) {
         const double fi = f2[scratch[i]];
@@ -184,7 +277,7 @@ __global__ void __launch_bounds__(1024) sort_slots_kernel(int32_t *order, const 
             const double fj = f2[scratch[j]];
             r += (fj < fi) || (fj == fi && j < i);
         }
-        order[r] = scratch[i];
+        (r < na ? a[r] : b[r - na]) = scratch[i];
     }
 }
 
@@ -635,6 +728,12 @@ void fill_const(const hea_problem *pb, uint64_t seed, SearchConst &c, PadGeom &g
     fill_lattice_const(pb, c);
 }
 
+// Site-histogram bytes of `slots` slots.
+size_t hist_bytes_of(const SearchConst &c, int64_t slots)
+{
+    return (size_t)slots * c.num_sites * sizeof(uint4);
+}
+
 // Whether a structure streams its histogram loads (SearchConst::hist_stream).
 // `total_bytes` is the histogram memory of every structure resident with it
 // (its own alone for a plan).  Until that total passes twice the L2 size the
@@ -850,9 +949,14 @@ struct hea_plan {
     DeviceTables dt;
     hea_params prm{};
     int P = 0;
-    cudaStream_t stream = nullptr, side = nullptr;  // side: the next iteration's new population
+    cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    std::vector<cudaEvent_t> joins;  // fork/join events between the two streams
+    Queue own;  // stream, ev0, ev1
+    // new populations searched ahead of the survivors (plan_lookahead): population r lives in slots
+    // order[P (r + 1), P (r + 2)) and is generated and searched on a stream of its own; events: its
+    // slots may be rewritten, its search has ended
+    enum { kFree, kDone };
+    std::vector<Queue> ahead;
     uint8_t *occ = nullptr, *out_occ = nullptr;
     int32_t *cnt = nullptr, *order = nullptr, *scratch = nullptr;
     double *f2 = nullptr, *out_f2 = nullptr;
@@ -869,20 +973,24 @@ struct hea_plan {
     };
     double *log_host = nullptr, *log_dev = nullptr;
     std::vector<LogEntry> log_entries;
-    ~hea_plan()
+    void free_buffers()
     {
-        if (stream) cudaStreamSynchronize(stream);  // buffers return to the pool only when idle
-        if (side) cudaStreamSynchronize(side);
-        if (log_host) cudaFreeHost(log_host);
-        for (cudaEvent_t e : mc_events) cudaEventDestroy(e);
-        for (cudaEvent_t e : joins) cudaEventDestroy(e);
-        if (side) cudaStreamDestroy(side);
         for (void *p : {(void *)occ, (void *)out_occ, (void *)cnt, (void *)order, (void *)scratch, (void *)f2,
                         (void *)out_f2, (void *)stats, (void *)hist})
             dev_free(p);
-        if (ev0) cudaEventDestroy(ev0);
-        if (ev1) cudaEventDestroy(ev1);
-        if (stream) cudaStreamDestroy(stream);
+        occ = out_occ = nullptr;
+        cnt = order = scratch = nullptr;
+        f2 = out_f2 = nullptr;
+        stats = nullptr;
+        hist = nullptr;
+    }
+    ~hea_plan()
+    {
+        queue_give(own);  // buffers return to the pool only when idle
+        for (Queue &q : ahead) queue_give(q);
+        if (log_host) cudaFreeHost(log_host);
+        for (cudaEvent_t e : mc_events) cudaEventDestroy(e);
+        free_buffers();
     }
 };
 
@@ -967,39 +1075,53 @@ int launch_mc(hea_plan *pl, const int32_t *order, int count, uint32_t mc_call, M
     return HEA_OK;
 }
 
-int launch_sort(hea_plan *pl, int32_t *order, int count)
+// Stable sort by f2 of the survivors (order[0, P)) or, with `r`, of the
+// survivors followed by new population r: the merge, which leaves the best P
+// as survivors and the rest as population r's free slots.
+int launch_sort(hea_plan *pl, int r = -1)
 {
-    sort_slots_kernel<<<1, 1024, 0, pl->stream>>>(order, pl->f2, count, pl->scratch);
+    sort_slots_kernel<<<1, 1024, 0, pl->stream>>>(pl->order, pl->P, pl->order + (size_t)pl->P * (r + 1),
+                                                  r < 0 ? 0 : pl->P, pl->f2, pl->scratch);
     HEA_CUDA(cudaGetLastError());
+    return HEA_OK;
+}
+
+int plan_streams(hea_plan *pl, int ahead)
+{
+    // the survivors' searches are the chain every iteration waits for: their CTAs start before the
+    // waiting ones of the populations searched ahead
+    HEA_TRY(queue_take(true, &pl->own));
+    pl->stream = pl->own.stream;
+    pl->ev0 = pl->own.ev[0];
+    pl->ev1 = pl->own.ev[1];
+    pl->ahead.resize(ahead);
+    for (Queue &q : pl->ahead) HEA_TRY(queue_take(false, &q));
     return HEA_OK;
 }
 
 int plan_alloc(hea_plan *pl, int slots)
 {
     const SearchConst &c = pl->dt.c;
-    HEA_CUDA(cudaStreamCreateWithFlags(&pl->stream, cudaStreamNonBlocking));
-    HEA_CUDA(cudaStreamCreateWithFlags(&pl->side, cudaStreamNonBlocking));
-    for (int i = 0; i < 2; ++i) {
-        cudaEvent_t e;
-        HEA_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        pl->joins.push_back(e);
-    }
-    HEA_CUDA(cudaEventCreate(&pl->ev0));
-    HEA_CUDA(cudaEventCreate(&pl->ev1));
     const size_t occ_bytes = (size_t)slots * c.occ_stride;
     if (dev_alloc(&pl->occ, occ_bytes) != cudaSuccess ||
         dev_alloc(&pl->cnt, (size_t)slots * pl->dt.ncount * sizeof(int32_t)) != cudaSuccess ||
         dev_alloc(&pl->order, (size_t)slots * sizeof(int32_t)) != cudaSuccess ||
         dev_alloc(&pl->scratch, (size_t)slots * sizeof(int32_t)) != cudaSuccess ||
         dev_alloc(&pl->f2, (size_t)slots * sizeof(double)) != cudaSuccess ||
-        dev_alloc(&pl->out_occ, (size_t)slots * c.num_sites) != cudaSuccess ||
-        dev_alloc(&pl->out_f2, (size_t)slots * sizeof(double)) != cudaSuccess ||
+        dev_alloc(&pl->out_occ, (size_t)pl->P * c.num_sites) != cudaSuccess ||
+        dev_alloc(&pl->out_f2, (size_t)pl->P * sizeof(double)) != cudaSuccess ||
         dev_alloc(&pl->stats, 4 * sizeof(unsigned long long)) != cudaSuccess)
         return fail(HEA_ERR_NOMEM, "cannot allocate the population buffers (%zu bytes of occupancy)", occ_bytes);
-    if (dev_alloc(&pl->hist, (size_t)slots * c.num_sites * sizeof(uint4)) != cudaSuccess)
-        return fail(HEA_ERR_NOMEM, "cannot allocate the site histograms (%zu bytes)",
-                    (size_t)slots * c.num_sites * sizeof(uint4));
-    HEA_CUDA(cudaMemsetAsync(pl->occ, 0, occ_bytes, pl->stream));
+    const size_t hist_bytes = hist_bytes_of(c, slots);
+    if (dev_alloc(&pl->hist, hist_bytes) != cudaSuccess)
+        return fail(HEA_ERR_NOMEM, "cannot allocate the site histograms (%zu bytes)", hist_bytes);
+    return HEA_OK;
+}
+
+// Defined occupancy rows and the slots in order.
+int plan_clear(hea_plan *pl, int slots)
+{
+    HEA_CUDA(cudaMemsetAsync(pl->occ, 0, (size_t)slots * pl->dt.c.occ_stride, pl->stream));
     iota_kernel<<<(slots + 255) / 256, 256, 0, pl->stream>>>(pl->order, slots);
     HEA_CUDA(cudaGetLastError());
     return HEA_OK;
@@ -1062,6 +1184,12 @@ int read_population(hea_plan *pl, int count, uint8_t *out_occ, double *out_fitne
 // The global loop of accelerate.cpp:737-761: generation 0, then per iteration a
 // new population searched (call 2*it), merged (stable, current first), and the
 // survivors searched (call 2*it+1) and sorted.
+//
+// A new population's structures depend on nothing but the seed, so those of the
+// next iterations are generated and searched ahead, each on a stream of its
+// own, while an iteration's last searches, its merge and its survivors' search
+// run (plan_lookahead says how many).  Iteration it merges population it mod W
+// and thereby frees W's slots for iteration it + W's.
 int plan_search(hea_plan *pl, hea_stats *stats)
 {
     const int P = pl->P;
@@ -1074,38 +1202,34 @@ int plan_search(hea_plan *pl, hea_stats *stats)
         }
     }
     HEA_TRY(plan_log_buffers(pl));
+    const int I = pl->prm.total_iter, W = (int)pl->ahead.size(), slots = P * (W + 1);
     HEA_CUDA(cudaMemsetAsync(pl->stats, 0, 4 * sizeof(unsigned long long), pl->stream));
-    iota_kernel<<<(2 * P + 255) / 256, 256, 0, pl->stream>>>(pl->order, 2 * P);
+    iota_kernel<<<(slots + 255) / 256, 256, 0, pl->stream>>>(pl->order, slots);
     HEA_CUDA(cudaGetLastError());
     HEA_CUDA(cudaEventRecord(pl->ev0, pl->stream));
+    // generation it + 1 and its local search, in population it mod W once its slots are free
+    const auto start_population = [pl, P, W](int it) -> int {
+        Queue &a = pl->ahead[it % W];
+        int32_t *order = pl->order + (size_t)P * (it % W + 1);
+        HEA_CUDA(cudaEventRecord(a.ev[hea_plan::kFree], pl->stream));
+        HEA_CUDA(cudaStreamWaitEvent(a.stream, a.ev[hea_plan::kFree], 0));
+        HEA_TRY(launch_generate(pl, order, P, (uint32_t)(it + 1), 1, a.stream));
+        HEA_TRY(launch_mc(pl, order, P, (uint32_t)(2 * it), McArgs{}, a.stream));
+        HEA_CUDA(cudaEventRecord(a.ev[hea_plan::kDone], a.stream));
+        return HEA_OK;
+    };
+    for (int it = 0; it < std::min(I, W); ++it) HEA_TRY(start_population(it));
     HEA_TRY(launch_generate(pl, pl->order, P, 0, 1));
-    const int I = pl->prm.total_iter;
-    if (I > 0) {
-        HEA_TRY(launch_generate(pl, pl->order + P, P, 1, 1));
-        HEA_TRY(launch_mc(pl, pl->order + P, P, 0, McArgs{}));
-        HEA_TRY(launch_sort(pl, pl->order, 2 * P));
-    }
     for (int it = 0; it < I; ++it) {
-        // after the merge of iteration it, the new population of iteration it+1
-        // (free slots order[P, 2P)) is generated and searched on the side stream
-        // while the survivors (order[0, P)) are searched on the main stream
-        if (it + 1 < I) {
-            HEA_CUDA(cudaEventRecord(pl->joins[0], pl->stream));
-            HEA_CUDA(cudaStreamWaitEvent(pl->side, pl->joins[0], 0));
-            HEA_TRY(launch_generate(pl, pl->order + P, P, (uint32_t)(it + 2), 1, pl->side));
-            HEA_TRY(launch_mc(pl, pl->order + P, P, (uint32_t)(2 * (it + 1)), McArgs{}, pl->side));
-            HEA_CUDA(cudaEventRecord(pl->joins[1], pl->side));
-        }
+        HEA_CUDA(cudaStreamWaitEvent(pl->stream, pl->ahead[it % W].ev[hea_plan::kDone], 0));
+        HEA_TRY(launch_sort(pl, it % W));  // the merge
+        if (it + W < I) HEA_TRY(start_population(it + W));
         HEA_TRY(launch_mc(pl, pl->order, P, (uint32_t)(2 * it + 1), McArgs{}));
-        HEA_TRY(launch_sort(pl, pl->order, P));
+        HEA_TRY(launch_sort(pl));
         if (pl->prm.flags & HEA_FLAG_LOG_ITERS) {  // the reference's per-iteration line (accelerate.cu:1208-1212)
             best_f2_kernel<<<1, 1, 0, pl->stream>>>(pl->order, pl->f2, pl->log_dev + it);
             HEA_CUDA(cudaGetLastError());
             HEA_CUDA(cudaLaunchHostFunc(pl->stream, log_callback, &pl->log_entries[it]));
-        }
-        if (it + 1 < I) {
-            HEA_CUDA(cudaStreamWaitEvent(pl->stream, pl->joins[1], 0));
-            HEA_TRY(launch_sort(pl, pl->order, 2 * P));  // merge of iteration it+1
         }
     }
     HEA_CUDA(cudaEventRecord(pl->ev1, pl->stream));
@@ -1236,6 +1360,43 @@ int plan_autotune(hea_plan *pl, bool measure)
     return HEA_OK;
 }
 
+// How many new populations a search keeps in flight beside its survivors.  One
+// leaves the chip waiting for each iteration's slowest searches, merge and
+// survivors, and a population smaller than the chip never fills it; enough of
+// them keep two chips' worth of CTAs queued.  Bounded by the iterations, by
+// kMaxAhead streams and by kAheadBytes of population buffers beyond the first.
+// Measured on B200, one population in flight -> this rule, whole call or run:
+// FCC 10^3 (128 solutions x 256 tasks, 10 iterations) 9.64 -> 3.77 ms, a
+// 5148-site box (48 x 200, 6 iterations) 5.23 -> 2.17 ms, BCC 20^3 (256 x 512,
+// 8 iterations; its 256 CTAs nearly fill the chip alone) 45.3 -> 37.7 ms.
+constexpr int kMaxAhead = 16;
+constexpr size_t kAheadBytes = (size_t)4 << 30;
+
+int plan_lookahead(const hea_plan *pl, int *out)
+{
+    const DeviceTables &dt = pl->dt;
+    const hea_params &prm = pl->prm;
+    *out = 1;
+    if (prm.total_iter < 2) return HEA_OK;
+    int dev = 0, sms = 0, per_sm = 1;
+    HEA_CUDA(cudaGetDevice(&dev));
+    HEA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (dt.large) {  // 512-thread CTAs, two per SM, a cluster of up to 8 per solution
+        const int csize = std::min(8, std::max(1, (prm.parallel_task + 511) / 512));
+        sms = 2 * sms / csize;
+    } else {
+        HEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &per_sm, dt.mc, pl->mc_block, mc_smem(dt.c.occ_stride, dt.T, dt.S, pl->mc_block / 32)));
+    }
+    const int64_t want = (2 * (int64_t)sms * std::max(1, per_sm) + pl->P - 1) / pl->P;
+    const size_t each = (hist_bytes_of(dt.c, 1) + dt.c.occ_stride) * (size_t)pl->P;
+    const int64_t room = 1 + (int64_t)(kAheadBytes / each);
+    *out = (int)std::max<int64_t>(1, std::min<int64_t>({std::max<int64_t>(2, want), room, kMaxAhead, prm.total_iter}));
+    return HEA_OK;
+}
+
+// `slots`: the plan's slots; 0 for a whole search, whose survivors and
+// populations ahead set them.
 int plan_create(const hea_problem *pb, const hea_params *prm, int slots, hea_plan **out)
 {
     *out = nullptr;
@@ -1246,8 +1407,19 @@ int plan_create(const hea_problem *pb, const hea_params *prm, int slots, hea_pla
         pl->prm = *prm;
         pl->P = prm->num_solutions;
         pl->mc_block = choose_block(prm->parallel_task);
-        rc = plan_alloc(pl, slots);
-        const size_t hist_bytes = (size_t)slots * pl->dt.N * sizeof(uint4);
+        int ahead = 0;
+        if (slots == 0) rc = plan_lookahead(pl, &ahead);
+        if (rc == HEA_OK) rc = plan_alloc(pl, slots ? slots : pl->P * (ahead + 1));
+        while (slots == 0 && rc == HEA_ERR_NOMEM && ahead > 1) {  // less memory than that: fewer ahead
+            ahead = (ahead + 1) / 2;
+            cudaGetLastError();
+            pl->free_buffers();
+            rc = plan_alloc(pl, pl->P * (ahead + 1));
+        }
+        if (rc == HEA_OK) rc = plan_streams(pl, ahead);
+        if (slots == 0) slots = pl->P * (ahead + 1);
+        if (rc == HEA_OK) rc = plan_clear(pl, slots);
+        const size_t hist_bytes = hist_bytes_of(pl->dt.c, slots);
         pl->dt.c.hist_stream = stream_histograms(hist_bytes, hist_bytes);
     }
     if (rc == HEA_OK) rc = plan_autotune(pl, (prm->flags & HEA_FLAG_AUTOTUNE) != 0);
@@ -1285,6 +1457,14 @@ void hea_release_cached_memory(void)
     DevicePool &P = pool();
     std::lock_guard<std::mutex> lk(P.mu);
     pool_release_device(P, dev);
+    const CUcontext ctx = current_context();
+    QueuePool &Q = queue_pool();
+    std::lock_guard<std::mutex> lq(Q.mu);
+    for (size_t i = Q.kept.size(); i-- > 0;)
+        if (Q.kept[i].ctx == ctx) {
+            queue_destroy(Q.kept[i]);
+            Q.kept.erase(Q.kept.begin() + i);
+        }
 }
 
 int hea_cuda_available(void)
@@ -1425,7 +1605,7 @@ int hea_plan_create(const hea_problem *problem, const hea_params *params, hea_pl
 {
     if (!out) return fail(HEA_ERR_INVALID, "out is NULL");
     HEA_TRY(validate_params(params));
-    return plan_create(problem, params, 2 * params->num_solutions, out);
+    return plan_create(problem, params, 0, out);
 }
 
 int hea_plan_run(hea_plan *plan, uint64_t seed, hea_stats *stats)
@@ -1785,7 +1965,7 @@ extern "C" int hea_recount_noalloc(const hea_problem *problem, int32_t count, co
 // ---------------------------------------------------------------------------
 // Batched search: many structures in one persistent kernel (hea_batch.cuh)
 // ---------------------------------------------------------------------------
-#include "hea_batch.cuh"
+#include "hea_batch.h"
 
 namespace {
 struct BatchLevels {
@@ -1885,7 +2065,7 @@ int batch_smem_budget(size_t *out, int ctas_per_sm = HEA_BATCH_MIN_BLOCKS)
 {
     cudaFuncAttributes a;
     int dev = 0, per_sm = 0, reserved = 0;
-    HEA_CUDA(cudaFuncGetAttributes(&a, batch_kernel));
+    HEA_CUDA(cudaFuncGetAttributes(&a, batch_kernel_fn()));
     HEA_CUDA(cudaGetDevice(&dev));
     HEA_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
     HEA_CUDA(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
@@ -1913,12 +2093,12 @@ int batch_configure(hea_batch *b, int hbm_all, int ctas_per_sm)
         smem = std::max(smem, batch_job_smem(d.c.occ_stride, T, S, nwarps, d.hbm != 0));
     }
     cudaFuncAttributes a;
-    HEA_CUDA(cudaFuncGetAttributes(&a, batch_kernel));
+    HEA_CUDA(cudaFuncGetAttributes(&a, batch_kernel_fn()));
     if (smem + a.sharedSizeBytes > (size_t)smem_limit())
         return fail(HEA_ERR_UNSUPPORTED, "the largest structure needs %zu bytes of shared memory, above %d", smem,
                     smem_limit() - (int)a.sharedSizeBytes);
     int per_sm = 0, sms = 0, dev = 0;
-    HEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel, b->block, smem));
+    HEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel_fn(), b->block, smem));
     HEA_CUDA(cudaGetDevice(&dev));
     HEA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     per_sm = std::min(per_sm, ctas_per_sm);
@@ -1936,8 +2116,8 @@ int batch_configure(hea_batch *b, int hbm_all, int ctas_per_sm)
     // the run as one CUDA graph: reset the queue, seed phase 0, persistent kernel
     HEA_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     batch_reset_kernel<<<64, 256, 0, b->stream>>>(b->d_ctl, b->d_jobs, b->total_jobs, *b->lv, b->wait_limit_ns);
-    batch_seed_kernel<<<b->count, 256, 0, b->stream>>>(b->d_structs, nullptr, b->d_states, b->d_jobs, b->d_ctl);
-    batch_kernel<<<b->grid, b->block, b->smem, b->stream>>>(b->d_structs, b->d_states, b->d_jobs, b->d_ctl,
+    batch_seed_kernel_fn()<<<b->count, 256, 0, b->stream>>>(b->d_structs, nullptr, b->d_states, b->d_jobs, b->d_ctl);
+    batch_kernel_fn()<<<b->grid, b->block, b->smem, b->stream>>>(b->d_structs, b->d_states, b->d_jobs, b->d_ctl,
                                                             b->d_finish);
     HEA_CUDA(cudaStreamEndCapture(b->stream, &b->graph));
     HEA_CUDA(cudaGraphInstantiate(&b->exec, b->graph, 0));
@@ -1957,9 +2137,6 @@ int hea_batch_create(const hea_problem *problems, const hea_params *params, int3
     if (!b) return fail(HEA_ERR_NOMEM, "out of host memory");
     b->count = count;
     size_t hist_total = 0;  // site-histogram bytes of all structures (stream_histograms)
-    for (int i = 0; i < count; ++i)
-        hist_total += (size_t)2 * std::max(0, params[i].num_solutions) * std::max(0, problems[i].num_sites) *
-                      sizeof(uint4);
     int rc = HEA_OK;
     for (int i = 0; i < count && rc == HEA_OK; ++i) {
         rc = validate_params(&params[i]);
@@ -1979,7 +2156,7 @@ int hea_batch_create(const hea_problem *problems, const hea_params *params, int3
         const int P = params[i].num_solutions, slots = 2 * P;
         BatchStruct d{};
         d.c = t->c;
-        d.c.hist_stream = stream_histograms((size_t)slots * t->N * sizeof(uint4), hist_total);
+        hist_total += hist_bytes_of(d.c, slots);
         d.nbor = t->nbor;
         d.P = P;
         d.Q = params[i].parallel_task;
@@ -1994,7 +2171,7 @@ int hea_batch_create(const hea_problem *problems, const hea_params *params, int3
         if ((rc = batch_alloc(b, &d.f2, (size_t)slots * sizeof(double))) != HEA_OK) break;
         if ((rc = batch_alloc(b, &d.order, (size_t)slots * sizeof(int32_t))) != HEA_OK) break;
         if ((rc = batch_alloc(b, &d.scratch, (size_t)slots * sizeof(int32_t))) != HEA_OK) break;
-        if ((rc = batch_alloc(b, &d.hist, (size_t)slots * t->N * sizeof(uint4))) != HEA_OK) break;
+        if ((rc = batch_alloc(b, &d.hist, hist_bytes_of(d.c, slots))) != HEA_OK) break;
         d.nbmask = t->nbmask;
         if (cudaMemset(d.occ, 0, (size_t)slots * t->c.occ_stride) != cudaSuccess) {
             rc = fail(HEA_ERR_CUDA, "cudaMemset failed");
@@ -2003,6 +2180,7 @@ int hea_batch_create(const hea_problem *problems, const hea_params *params, int3
         b->h_structs.push_back(d);
         b->total_jobs += d.I > 0 ? (unsigned long long)P * (2 * d.I + 1) : (unsigned long long)P;
     }
+    for (BatchStruct &d : b->h_structs) d.c.hist_stream = stream_histograms(hist_bytes_of(d.c, 2 * d.P), hist_total);
     // priority levels: structures ranked by work, largest first
     BatchLevels lv{};
     if (rc == HEA_OK) {
@@ -2038,7 +2216,7 @@ int hea_batch_create(const hea_problem *problems, const hea_params *params, int3
         cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreate(&b->ev0);
         if (e == cudaSuccess) e = cudaEventCreate(&b->ev1);
-        if (e == cudaSuccess) e = allow_max_smem(batch_kernel);
+        if (e == cudaSuccess) e = allow_max_smem(batch_kernel_fn());
         if (e != cudaSuccess) rc = fail(HEA_ERR_CUDA, "batch set-up failed: %s", cudaGetErrorString(e));
     }
     // Occupancy in HBM by default: with site-histogram scoring a search reads it
@@ -2284,7 +2462,7 @@ RequestLayout request_layout(const SearchConst &c, int64_t pad_row, int S, int T
     };
     L.nbor = take((size_t)c.num_sites * pad_row * sizeof(int32_t));
     L.nbmask = take(nbmask_words(c.num_sites) * sizeof(uint32_t));
-    L.hist = take(slots * c.num_sites * sizeof(uint4));
+    L.hist = take(hist_bytes_of(c, (int64_t)slots));
     L.occ = take(slots * c.occ_stride);
     L.cnt = take(slots * (size_t)S * T * T * sizeof(int32_t));
     L.f2 = take(slots * sizeof(double));
@@ -2449,7 +2627,7 @@ int server_place(hea_server *sv, ServerRequest &r, int slot)
     }
     BatchStruct d{};
     d.c = c;
-    r.hist_bytes = (size_t)2 * P * r.N * sizeof(uint4);
+    r.hist_bytes = hist_bytes_of(c, 2 * (int64_t)P);
     sv->hist_placed += r.hist_bytes;
     d.c.hist_stream = stream_histograms(r.hist_bytes, sv->hist_placed);
     d.nbor = implicit ? nullptr : reinterpret_cast<const int4 *>(base + L.nbor);
@@ -2541,7 +2719,7 @@ int server_admit(hea_server *sv)
     if (sv->h_list.empty()) return HEA_OK;
     HEA_CUDA(cudaMemcpyAsync(sv->d_list, sv->h_list.data(), sizeof(int32_t) * sv->h_list.size(),
                              cudaMemcpyHostToDevice, sv->stream));
-    batch_seed_kernel<<<(unsigned)sv->h_list.size(), 256, 0, sv->stream>>>(sv->d_structs, sv->d_list, sv->d_states,
+    batch_seed_kernel_fn()<<<(unsigned)sv->h_list.size(), 256, 0, sv->stream>>>(sv->d_structs, sv->d_list, sv->d_states,
                                                                              sv->d_jobs, sv->d_ctl);
     HEA_CUDA(cudaGetLastError());
     return HEA_OK;
@@ -2708,7 +2886,7 @@ int hea_server_create(const hea_server_config *config, hea_server **out)
         sv->smem = cfg.smem_bytes > 0 ? (size_t)cfg.smem_bytes : (cfg.hbm_sites == 0 ? least : budget);
         sv->smem = std::max(sv->smem, least);
         cudaFuncAttributes a;
-        if (cudaFuncGetAttributes(&a, batch_kernel) != cudaSuccess) rc = fail(HEA_ERR_CUDA, "cannot query the batch kernel");
+        if (cudaFuncGetAttributes(&a, batch_kernel_fn()) != cudaSuccess) rc = fail(HEA_ERR_CUDA, "cannot query the batch kernel");
         else if (sv->smem + a.sharedSizeBytes > (size_t)smem_limit())
             rc = fail(HEA_ERR_INVALID, "smem_bytes %zu above the device limit", sv->smem);
         cfg.smem_bytes = (int32_t)sv->smem;
@@ -2729,10 +2907,10 @@ int hea_server_create(const hea_server_config *config, hea_server **out)
         sv->h_err.assign(M, 0);
         sv->slot_req.assign(M, 0);
         sv->h_list.reserve(M);
-        cudaError_t e = allow_max_smem(batch_kernel);
+        cudaError_t e = allow_max_smem(batch_kernel_fn());
         int per_sm = 0, sms = 0, dev = 0;
         if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel, HEA_BATCH_THREADS, sv->smem);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel_fn(), HEA_BATCH_THREADS, sv->smem);
         if (e == cudaSuccess) e = cudaGetDevice(&dev);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (e == cudaSuccess) e = cudaMallocHost((void **)&sv->h_states, sizeof(BatchState) * M);
@@ -2866,7 +3044,7 @@ int hea_server_step(hea_server *server, int32_t *out_finished)
     if (sv->running > 0) {
         HEA_CUDA(cudaEventRecord(sv->ev0, sv->stream));
         server_arm_kernel<<<1, 1, 0, sv->stream>>>(sv->d_ctl, (unsigned long long)(sv->cfg.slice_ms * 1e6));
-        batch_kernel<<<sv->grid, HEA_BATCH_THREADS, sv->smem, sv->stream>>>(sv->d_structs, sv->d_states,
+        batch_kernel_fn()<<<sv->grid, HEA_BATCH_THREADS, sv->smem, sv->stream>>>(sv->d_structs, sv->d_states,
                                                                              sv->d_jobs, sv->d_ctl, sv->d_finish);
         HEA_CUDA(cudaGetLastError());
         HEA_CUDA(cudaEventRecord(sv->ev1, sv->stream));

@@ -1,0 +1,78 @@
+"""Populations searched ahead of the survivors: whole searches whose iterations
+outnumber the populations in flight (their slots are reused), plans run again
+and from several threads, and calls after the cached streams were given back,
+all equal to the oracle bit for bit."""
+import threading
+
+import numpy as np
+import pytest
+
+import pyhea_b200 as hb
+from oracle import hea_oracle as ho
+from pyhea_b200 import lattice as L
+from pyhea_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def case(seed, lattice=L.BCC, cell=3, species=(20, 17, 17)):
+    st = W.small_case(lattice=lattice, cell=cell, species=species, shells=2, seed=seed)
+    nbor, sizes = st.neighbors()
+    return (hb.Problem(nbor, sizes, st.species, st.weight, st.target),
+            ho.Problem(nbor, sizes, st.species, st.weight, st.target))
+
+
+def same(got, want):
+    occ, fit = got[0], got[1]
+    wocc, wf2 = want[0], want[1]
+    np.testing.assert_array_equal(occ, wocc)
+    np.testing.assert_array_equal(fit, np.sqrt(wf2))
+
+
+@pytest.mark.parametrize("iters", [1, 2, 16, 17, 35])
+def test_iterations_around_the_populations_in_flight(iters):
+    gp, op = case(iters)
+    same(hb.search(gp, 3, iters, 24, 3, seed=11 + iters), op.hcs(11 + iters, 3, iters, 24, 3))
+
+
+def test_cluster_path_reuses_population_slots():
+    gp, op = case(5)
+    same(hb.search(gp, 2, 19, 40, 2, seed=3, hbm_occupancy=True), op.hcs(3, 2, 19, 40, 2))
+
+
+def test_plan_runs_again():
+    gp, op = case(7)
+    plan = hb.Plan(gp, 4, 18, 16, 3)
+    for seed in (1, 2, 1):
+        plan.run(seed)
+        same(plan.read(), op.hcs(seed, 4, 18, 16, 3))
+    plan.close()
+
+
+def test_threads_share_the_stream_cache():
+    gp, op = case(9)
+    want = {s: op.hcs(s, 3, 4, 24, 3) for s in range(6)}
+    got, errors = {}, []
+
+    def work(s):
+        try:
+            for _ in range(4):
+                got[s] = hb.search(gp, 3, 4, 24, 3, seed=s)
+        except Exception as e:  # reported by the main thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in want]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    for s in want:
+        same(got[s], want[s])
+
+
+def test_after_release_of_cached_memory():
+    gp, op = case(13)
+    for _ in range(2):
+        same(hb.search(gp, 3, 3, 24, 3, seed=4), op.hcs(4, 3, 3, 24, 3))
+        hb.lib.hea_release_cached_memory()

@@ -130,16 +130,24 @@ struct JobEnd {
 };
 
 // One job of a structure with species count T and layout L.  Shared memory:
-// [occ5 (occ_stride + 16), unless hbm] | search_smem_tail(T, S, nwarps) (delta
+// [occ (occ_stride + 16), unless hbm] | search_smem_tail(T, S, nwarps) (delta
 // table, swap records, two count buffers).
 // The rounds of a job's local search in a call of their own: values the job
 // needs only before and after the search stay out of the loop's registers.
-template <int T, class L>
-__device__ __noinline__ McTally batch_search(const SearchConst &c, const BatchStruct &d, uint8_t *occ5, int32_t *cnt2,
-                                             double2 *tab, SwapRecord *rec, uint32_t stream, double cur,
-                                             const McResume rs, uint4 *hist)
+// One recount instance for the layouts that share it.
+template <int T, int S, RecountForm kNeighbors>
+__device__ __noinline__ void batch_recount(const SearchConst &c, const int4 *nbor, const uint8_t *occ, int32_t *cnt,
+                                           uint64_t *hist)
 {
-    return mc_rounds<T, L, true>(c, d.nbor, occ5, cnt2, tab, rec, stream, cur, d.Q, d.D, d.max_rounds,
+    block_recount<T, S, kNeighbors>(c, nbor, occ, cnt, hist);
+}
+
+template <int T, class L>
+__device__ __noinline__ McTally batch_search(const SearchConst &c, const BatchStruct &d, uint8_t *occ, int32_t *cnt2,
+                                             const DeltaTab<T, L::S> tab, void *rec, uint32_t stream, double cur,
+                                             const McResume rs, uint64_t *hist)
+{
+    return mc_rounds<T, L, false, true>(c, d.nbor, occ, cnt2, tab, rec, stream, cur, d.Q, d.D, d.max_rounds,
                                  McTrace{nullptr, nullptr, 0}, rs, hist, d.nbmask);
 }
 
@@ -156,28 +164,27 @@ __device__ __noinline__ JobEnd batch_job(const SearchConst &c, const BatchStruct
     const int slot = __ldcg(d.order + (job.kind == kJobGenMc ? P + pos : pos));
     uint8_t *gocc = d.occ + (size_t)slot * c.occ_stride;
     int32_t *gcnt = d.cnt + (size_t)slot * NC;
-    uint4 *hist = d.hist + (size_t)slot * c.num_sites;
-    uint8_t *occ5 = hbm ? gocc : smem;
-    double2 *tab = reinterpret_cast<double2 *>(hbm ? smem : smem + c.occ_stride + 16);
-    SwapRecord *rec = reinterpret_cast<SwapRecord *>(tab + delta_entries(T, S));
-    int32_t *cnt2 = reinterpret_cast<int32_t *>(rec + 2 * nwarps);
+    uint64_t *hist = d.hist + (size_t)slot * c.num_sites * hist_words(T, S, L::kImplicit);
+    uint8_t *occ = hbm ? gocc : smem;
+    const DeltaTab<T, S> tab{reinterpret_cast<float *>(hbm ? smem : smem + c.occ_stride + 16)};
+    uint8_t *rec = reinterpret_cast<uint8_t *>(tab.f + DeltaTab<T, S>::kFloats);  // [2][nwarps] records
+    int32_t *cnt2 = reinterpret_cast<int32_t *>(rec + 2 * nwarps * record_bytes(T, S));
 
     double cur;
     if (job.kind == kJobMc2 || job.resume) {
-        stage_occupancy<true>(c, gocc, occ5);  // in place when hbm
+        copy_occupancy<true>(c, gocc, occ);  // onto itself when hbm
         for (int x = threadIdx.x; x < NC; x += blockDim.x) cnt2[x] = __ldcg(gcnt + x);
         __syncthreads();
-        if (threadIdx.x == 0) occ5[n] = 0;  // sentinel
+        if (threadIdx.x == 0) occ[n] = 0;  // sentinel
         cur = __ldcg(d.f2 + slot);  // a resumed search's running f2
     } else {
         const uint32_t generation = job.kind == kJobGen0 ? 0u : (uint32_t)(job.iter + 1);
-        generate_occupancy<T>(c, (uint32_t)pos, generation, occ5, (job.kind == kJobGen0 && !hbm) ? gocc : nullptr);
-        if (threadIdx.x == 0) occ5[n] = 0;
+        generate_occupancy<T>(c, (uint32_t)pos, generation, occ, (job.kind == kJobGen0 && !hbm) ? gocc : nullptr);
+        if (threadIdx.x == 0) occ[n] = 0;
         __syncthreads();
-        block_recount<T, S>(c, d.nbor, occ5, cnt2, hist);  // count buffer 0; ends with a barrier
+        batch_recount<T, S, L::kImplicit ? kRecountLattice : kRecountTable>(c, d.nbor, occ, cnt2, hist);  // count buffer 0; ends with a barrier
         cur = fitness_of_counts<T, S>(c, cnt2);
         if (job.kind == kJobGen0) {
-            if (hbm) unstage_occupancy(c, occ5, gocc);
             for (int x = threadIdx.x; x < NC; x += blockDim.x) gcnt[x] = cnt2[x];
             if (threadIdx.x == 0) d.f2[slot] = cur;
             return JobEnd{0, 0, 0};
@@ -188,13 +195,13 @@ __device__ __noinline__ JobEnd batch_job(const SearchConst &c, const BatchStruct
     const uint32_t stream = (call << 16) | (uint32_t)pos;
     const McResume rs{job.resume ? (int64_t)job.round0 : 0, job.resume ? job.miss0 : 0, deadline, d.tol2};
     // the draws read the species from the occupancy: measured on the mixed batch, the histograms'
-    // species words (draw_pair_hist) were slower for every structure size
-    const McTally t = batch_search<T, L>(c, d, occ5, cnt2, tab, rec, stream, cur, rs, hist);
-    unstage_occupancy(c, occ5, gocc);  // in place when hbm
+    // species bits (draw_pair_hist) were slower for every structure size
+    const McTally t = batch_search<T, L>(c, d, occ, cnt2, tab, rec, stream, cur, rs, hist);
+    if (!hbm) copy_occupancy(c, occ, gocc);
     for (int x = threadIdx.x; x < NC; x += blockDim.x) gcnt[x] = cnt2[t.buf * NCP + x];
     add_tally(t, stats);
     add_tally(t, tally);
-    if (threadIdx.x == 0) d.f2[slot] = t.f2;  // recomputed from the counts, or the running f2 of a yielded search
+    if (threadIdx.x == 0) d.f2[slot] = t.f2;  // McTally::f2
     return JobEnd{t.yielded ? 1 : 0, (int32_t)t.round_end, t.miss};
 }
 

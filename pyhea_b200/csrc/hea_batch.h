@@ -38,11 +38,11 @@
 // error flag and every CTA returns.
 //
 // Occupancy in HBM (`hbm`, the default: proposals are scored from the site
-// histograms, so a search reads the occupancy only for its draws): a job
-// converts the row to 5*species in place (reads through L2, so no stale L1
-// line of another SM's writes is used; the conversion rewrites every byte this
-// CTA later reads), searches it through L1, and converts it back.  Otherwise
-// the row is staged in the launch's shared memory.
+// histograms, so a search reads the occupancy only for its draws): a job copies
+// the row onto itself (reads through L2, so no stale L1 line of another SM's
+// writes is used; the copy rewrites every byte this CTA later reads) and
+// searches it through L1.  Otherwise the row is staged in the launch's shared
+// memory.
 #pragma once
 #include <cstdint>
 
@@ -73,7 +73,7 @@ struct BatchStruct {
     double *f2;
     int32_t *order;    // [2P] slot ids
     int32_t *scratch;  // [2P] sort scratch
-    uint4 *hist;       // [2P][N] site histograms
+    uint64_t *hist;    // [2P][N] site histograms (SiteHist)
     const uint32_t *nbmask;
     int32_t P, Q, D, I;
     int64_t max_rounds;

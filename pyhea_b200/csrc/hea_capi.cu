@@ -626,8 +626,8 @@ void fill_lattice_const(const hea_problem *pb, SearchConst &c)
         lc.zoff[k] = e;
         lc.zsize[k] = sp.size[k];
     }
-    lc.inv_L = 1.0 / lc.L;
-    lc.inv_LL = 1.0 / ((double)lc.L * lc.L);
+    lc.mul_L = (uint32_t)(0x100000000ull / (uint64_t)lc.L);
+    lc.mul_LL = (uint32_t)(0x100000000ull / ((uint64_t)lc.L * lc.L));
     lc.kind = pb->implicit_lattice == 2 ? kLatBcc : pb->lattice_shell_set == 1 ? kLatFccTrue3 : kLatFccRef;
     for (int k = 0; k < kMaxShells; ++k) c.pad[k] = 0;  // no sentinel padding in computed rows
 }
@@ -666,6 +666,24 @@ int choose_block(int tasks)
     return b;
 }
 
+// Threads per CTA of a plan's local search.  One task per thread (up to 512)
+// keeps a round shortest; a search with more solutions in flight (`ctas`, over
+// the populations ahead) than the four 256-thread CTAs an SM holds runs faster
+// with smaller CTAs that take a round in equal passes of at most 256 tasks,
+// since four CTAs hide each other's barriers and share each round's fixed work
+// over twice the tasks.  Measured, 512 -> 256 threads at 512 tasks: BCC 20^3, 256
+// solutions x 8 iterations 38.3 -> 30.0 ms; BCC 16^3, 300 x 2 2.53 -> 2.30 ms;
+// below the line 74 x 8 2.43 -> 2.55 ms, 148 x 2 1.40 -> 1.94 ms.
+int choose_plan_block(int tasks, int64_t ctas)
+{
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (tasks <= 256 || ctas <= 4 * (int64_t)sms) return choose_block(tasks);
+    const int passes = (tasks + 255) / 256;
+    return choose_block((tasks + passes - 1) / passes);
+}
+
 // Kernels are shared by every plan and batch: allow them the device's largest
 // dynamic shared memory (the opt-in limit less their static shared memory),
 // never one plan's size.
@@ -676,6 +694,40 @@ cudaError_t allow_max_smem(F *func)
     cudaError_t e = cudaFuncGetAttributes(&a, func);
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_limit() - (int)a.sharedSizeBytes);
+}
+
+// Constants of the FP32 screening (score_delta): its scale, and whether its
+// bound holds -- every Q and Cq at most about 1 and far above FP32's smallest
+// normal number, or zero, and no target so large that an L leaves its range.
+// (With |E| <= 1e6 an L stays below (|E| + N) / R_max < 1e20.)
+void fill_screen_const(const hea_problem *pb, SearchConst &c)
+{
+    const int T = pb->num_types, S = pb->num_shells;
+    double qmax = 0.0, qmin = HUGE_VAL, emax = 0.0;
+    for (int k = 0; k < S; ++k)
+        for (int e = 0; e < T * T; ++e) {
+            const double q = 2.0 * c.w[k] * c.R[k * T * T + e] * c.R[k * T * T + e];
+            if (q > 0.0) {
+                qmax = std::max(qmax, 2.0 * q);
+                qmin = std::min(qmin, q);
+            }
+            if (c.w[k] > 0.0) qmin = std::min(qmin, q);  // an underflow to 0
+            emax = std::max(emax, std::fabs(c.E[k * T * T + e]));
+        }
+    int exponent = 0;
+    if (qmax > 0.0 && std::isfinite(qmax)) std::frexp(qmax, &exponent);
+    c.screen_scale = std::ldexp(1.0, -exponent);
+    const bool fits = std::isfinite(qmax) && std::isfinite(c.screen_scale) && c.screen_scale > 0.0 && emax <= 1e6 &&
+                       (qmax == 0.0 || qmin * c.screen_scale >= std::ldexp(1.0, -100))
+;
+    c.screen_floor = fits ? 0.0f : kNoSwap;
+    if (!fits) c.screen_scale = 0.0;
+    for (int k = 0; k < S; ++k)
+        c.screen_sw[k] = std::nextafter((float)std::sqrt(c.w[k] * c.screen_scale), HUGE_VALF);
+    for (int i = 0; i < T; ++i)
+        for (int t = 0; t < T; ++t)
+            c.kappa[i * T + t] = std::nextafter(
+                (float)std::max(1.0, (double)pb->species[t] / (double)pb->species[i]), HUGE_VALF);
 }
 
 // Search constants and padded-table geometry of a validated problem.
@@ -709,9 +761,8 @@ void fill_const(const hea_problem *pb, uint64_t seed, SearchConst &c, PadGeom &g
     c.num_shells = S;
     c.occ_stride = (N + 1 + 15) & ~15;  // room for the sentinel byte N in HBM rows too
     c.feistel_h = feistel_half_bits((uint32_t)N);
-    c.reject_below = (uint32_t)(0u - (uint32_t)N) % (uint32_t)N;
     c.draw16 = use_draw16((uint32_t)N) ? 1u : 0u;
-    c.reject16 = c.draw16 ? 65536u % (uint32_t)N : 0u;
+    c.reject = c.draw16 ? (65536u % (uint32_t)N) << 16 : (uint32_t)(0u - (uint32_t)N) % (uint32_t)N;
     c.key0 = (uint32_t)seed;
     c.key1 = (uint32_t)(seed >> 32);
     c.prefix[0] = 0;
@@ -725,13 +776,14 @@ void fill_const(const hea_problem *pb, uint64_t seed, SearchConst &c, PadGeom &g
                 c.R[e] = (double)N / (((double)pb->shell_sizes[k] * (double)pb->species[i]) * (double)pb->species[j]);
             }
     }
+    fill_screen_const(pb, c);
     fill_lattice_const(pb, c);
 }
 
-// Site-histogram bytes of `slots` slots.
+// Site-histogram bytes of `slots` slots (SiteHist).
 size_t hist_bytes_of(const SearchConst &c, int64_t slots)
 {
-    return (size_t)slots * c.num_sites * sizeof(uint4);
+    return (size_t)slots * c.num_sites * hist_words(c.num_types, c.num_shells, c.lat.L > 0) * sizeof(uint64_t);
 }
 
 // Whether a structure streams its histogram loads (SearchConst::hist_stream).
@@ -739,8 +791,9 @@ size_t hist_bytes_of(const SearchConst &c, int64_t slots)
 // (its own alone for a plan).  Until that total passes twice the L2 size the
 // structures keep their lines cached; beyond it, those with more than
 // kSharedStreamBytes of their own stream, so that the lines of the smaller
-// ones stay.  Measured: a single 131 MB structure loses 3 % by streaming; on
-// the mixed batch (3.7 GB) thresholds of 4, 16 and 64 MiB are within 0.4 %.
+// ones stay.  Measured on batches of 8 FCC 30^3 structures (108 000
+// sites, 442 MB of histograms): 81.8 -> 74.2 ms (4 species), 94.6 -> 85.5 ms (6);
+// FCC 100^3 36.4 -> 35.0 ms.
 constexpr size_t kSharedStreamBytes = (size_t)64 << 20;
 
 uint32_t stream_histograms(size_t hist_bytes, size_t total_bytes)
@@ -960,7 +1013,7 @@ struct hea_plan {
     uint8_t *occ = nullptr, *out_occ = nullptr;
     int32_t *cnt = nullptr, *order = nullptr, *scratch = nullptr;
     double *f2 = nullptr, *out_f2 = nullptr;
-    uint4 *hist = nullptr;  // [slots][N] site histograms
+    uint64_t *hist = nullptr;  // [slots][N] site histograms
     unsigned long long *stats = nullptr;
     std::vector<cudaEvent_t> mc_events;  // start/stop pairs, HEA_FLAG_TIME_KERNELS
     int mc_timed = 0;
@@ -1053,7 +1106,7 @@ int launch_mc(hea_plan *pl, const int32_t *order, int count, uint32_t mc_call, M
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(count * csize);
         cfg.blockDim = dim3(block);
-        cfg.dynamicSmemBytes = search_smem_tail(pl->dt.T, pl->dt.S, nw) + 2 * sizeof(SwapRecord);
+        cfg.dynamicSmemBytes = search_smem_tail(pl->dt.T, pl->dt.S, nw) + 2 * record_bytes(pl->dt.T, pl->dt.S);
         cfg.stream = st;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1273,7 +1326,7 @@ int plan_search(hea_plan *pl, hea_stats *stats)
 // Autotuner of the local search's CTA size.  Every CTA size gives the same
 // result (the round's winner is the lexicographic (f2, task) minimum however
 // the tasks are split over warps and passes), so the choice is a pure speed
-// question: each candidate (the default one task per thread, and 256 and 128
+// question: each candidate (the default, choose_plan_block, and 256 and 128
 // threads when smaller) searches a fresh generation-0 population for
 // kTuneRounds rounds, once to warm up and kTunePasses times timed; a
 // candidate's rate is its best pass (evaluations per millisecond).  A smaller
@@ -1311,7 +1364,7 @@ int plan_autotune(hea_plan *pl, bool measure)
         }
     }
     if (!measure) return HEA_OK;
-    std::vector<int> cand = {choose_block(pl->prm.parallel_task)};
+    std::vector<int> cand = {pl->mc_block};  // choose_plan_block's
     for (int b : {256, 128})
         if (b < cand[0]) cand.push_back(b);
     int best = cand[0];
@@ -1406,7 +1459,8 @@ int plan_create(const hea_problem *pb, const hea_params *prm, int slots, hea_pla
     if (rc == HEA_OK) {
         pl->prm = *prm;
         pl->P = prm->num_solutions;
-        pl->mc_block = choose_block(prm->parallel_task);
+        pl->mc_block = choose_plan_block(prm->parallel_task,
+                                         (int64_t)prm->num_solutions * std::min(prm->total_iter, kMaxAhead));
         int ahead = 0;
         if (slots == 0) rc = plan_lookahead(pl, &ahead);
         if (rc == HEA_OK) rc = plan_alloc(pl, slots ? slots : pl->P * (ahead + 1));
@@ -1418,9 +1472,9 @@ int plan_create(const hea_problem *pb, const hea_params *prm, int slots, hea_pla
         }
         if (rc == HEA_OK) rc = plan_streams(pl, ahead);
         if (slots == 0) slots = pl->P * (ahead + 1);
-        if (rc == HEA_OK) rc = plan_clear(pl, slots);
         const size_t hist_bytes = hist_bytes_of(pl->dt.c, slots);
         pl->dt.c.hist_stream = stream_histograms(hist_bytes, hist_bytes);
+        if (rc == HEA_OK) rc = plan_clear(pl, slots);
     }
     if (rc == HEA_OK) rc = plan_autotune(pl, (prm->flags & HEA_FLAG_AUTOTUNE) != 0);
     if (rc != HEA_OK) {
@@ -2636,7 +2690,7 @@ int server_place(hea_server *sv, ServerRequest &r, int slot)
     d.f2 = reinterpret_cast<double *>(base + L.f2);
     d.order = reinterpret_cast<int32_t *>(base + L.order);
     d.scratch = reinterpret_cast<int32_t *>(base + L.scratch);
-    d.hist = reinterpret_cast<uint4 *>(base + L.hist);
+    d.hist = reinterpret_cast<uint64_t *>(base + L.hist);
     d.nbmask = reinterpret_cast<const uint32_t *>(base + L.nbmask);
     d.P = P;
     d.Q = r.params.parallel_task;

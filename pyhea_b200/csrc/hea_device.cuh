@@ -41,20 +41,10 @@ __host__ __device__ __forceinline__ u32x4 philox4x32_10(u32x4 c, uint32_t k0, ui
     return c;
 }
 
-// Lemire's multiply-and-reject bounded draw: exactly uniform on [0, n) when it accepts.
-__device__ __forceinline__ bool bounded_draw(uint32_t x, uint32_t n, uint32_t reject_below, uint32_t &v)
-{
-    v = __umulhi(x, n);
-    return x * n >= reject_below;
-}
-
-// The same on a 16-bit word h (n <= 2^16): accept iff low16(h n) >= 2^16 mod n; value high16(h n).
-__device__ __forceinline__ bool bounded_draw16(uint32_t h, uint32_t n, uint32_t reject16, uint32_t &v)
-{
-    const uint32_t m = h * n;
-    v = m >> 16;
-    return (m & 0xFFFFu) >= reject16;
-}
+// Bounded draws are Lemire's multiply-and-reject: x -> the high word of x * n,
+// rejected when the low word is below 2^32 mod n -- exactly uniform on [0, n).
+// The same on a 16-bit word h (n <= 2^16): high16(h n), rejected when low16(h n)
+// is below 2^16 mod n.
 
 // Whether proposals of a structure of n sites use 16-bit draws (four attempts
 // per Philox call): n <= 2^16 and at most 1/16 of the 16-bit words rejected.

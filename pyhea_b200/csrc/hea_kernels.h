@@ -9,7 +9,7 @@ namespace hea {
 using GenFn = void (*)(const SearchConst, const GenArgs);
 using McFn = void (*)(const SearchConst, const McArgs);
 using LGenFn = void (*)(const SearchConst, uint8_t *, const int32_t *, uint32_t);
-using LRecFn = void (*)(const SearchConst, const int4 *, const uint8_t *, const int32_t *, int32_t *, uint4 *);
+using LRecFn = void (*)(const SearchConst, const int4 *, const uint8_t *, const int32_t *, int32_t *, uint64_t *);
 using LFitFn = void (*)(const SearchConst, const int32_t *, int, const int32_t *, double *);
 
 struct KernelSet {

@@ -6,9 +6,9 @@
 // the occupancy lives and how many SMs work on one solution change:
 //   * the occupancy row stays in HBM as species bytes; the local search does
 //     not read or write it: its draws take the species from the site
-//     histograms' species words (hist[s].w = 5*species), which the accepts
+//     histograms' species bits, which the accepts
 //     keep current, and at its end each CTA writes its share of the row back
-//     from those words;
+//     from those bits;
 //   * one thread-block cluster per solution: the round's tasks are split over
 //     the cluster's CTAs; each CTA reduces its warps' records, publishes its
 //     best in shared memory, and after one cluster barrier every warp reads the
@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(256) large_generate_kernel(const SearchConst c
 template <int T, int S>
 __global__ void __launch_bounds__(256) large_recount_kernel(const SearchConst c, const int4 *__restrict__ nbor,
                                                             const uint8_t *occ, const int32_t *order, int32_t *cnt,
-                                                            uint4 *hist)
+                                                            uint64_t *hist)
 {
     __shared__ int32_t bins[S * T * T];
     const int slot = order[blockIdx.y];
@@ -66,11 +66,11 @@ __global__ void __launch_bounds__(256) large_recount_kernel(const SearchConst c,
     for (int x = threadIdx.x; x < S * T * T; x += blockDim.x) bins[x] = 0;
     __syncthreads();
     const int n = c.num_sites;
-    uint4 *hs = hist ? hist + (size_t)slot * n : nullptr;
+    uint64_t *hs = hist ? hist + (size_t)slot * n * hist_words(T, S, c.lat.L > 0) : nullptr;
     // one site with its shell histograms h (5-bit fields)
-    const auto site = [&](int s, const uint32_t (&h)[S]) {
+    const auto site = [&](int s, const uint32_t (&h)[S], auto form) {
+        using H = SiteHist<T, S, decltype(form)::value>;
         const int a = row[s];
-        uint32_t hk[3] = {0u, 0u, 0u};
 #pragma unroll
         for (int k = 0; k < S; ++k) {
 #pragma unroll
@@ -78,13 +78,17 @@ __global__ void __launch_bounds__(256) large_recount_kernel(const SearchConst c,
                 const int v = (int)((h[k] >> (5 * t)) & 31u);
                 if (v) atomicAdd(&bins[(k * T + a) * T + t], v);
             }
-            hk[k] = h[k] - (uint32_t)c.pad[k];  // sentinel entries counted as species 0
         }
-        if (hs) hs[s] = make_uint4(hk[0], hk[1], hk[2], (uint32_t)(5 * a));  // species word: 5*species
+        if (hs) {
+            const HistEntry<H::W> e = pack_hist<H, T, S, 5>(c, h, a);
+#pragma unroll
+            for (int x = 0; x < H::W; ++x) hs[(size_t)s * H::W + x] = e.w[x];
+        }
     };
     const int first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     if (c.lat.L) {  // implicit neighbours (no sentinel padding: pad[k] == 0)
-        lattice_sites<S, uint32_t>(c.lat, first, stride, [row](int n) { return 1u << (5 * row[n]); }, site);
+        lattice_sites<S, uint32_t>(c.lat, first, stride, [row](int n) { return 1u << (5 * row[n]); },
+                                   [&site](int s, const uint32_t (&h)[S]) { site(s, h, std::true_type{}); });
     } else {
         for (int s = first; s < n; s += stride) {
             uint32_t h[S];
@@ -98,7 +102,7 @@ __global__ void __launch_bounds__(256) large_recount_kernel(const SearchConst c,
                             (1u << (5 * row[x.w]));
                 }
             }
-            site(s, h);
+            site(s, h, std::false_type{});
         }
     }
     __syncthreads();
@@ -125,32 +129,35 @@ __global__ void large_fitness_kernel(const SearchConst c, const int32_t *order, 
 }
 
 // The local search with the occupancy in HBM, one cluster per solution.
-// Shared memory: search_smem_tail(T, S, nwarps) + 2 * sizeof(SwapRecord):
-// delta table, the warps' records [2][nwarps], two count buffers, and this
-// CTA's best record [2] (read by the cluster).  Every CTA keeps its own copy of
+// Shared memory: search_smem_tail(T, S, nwarps) + 2 * record_bytes(T, S):
+// delta table, the warps' records [2][nwarps], this CTA's best record [2]
+// (read by the cluster), and two count buffers.  Every CTA keeps its own copy of
 // the table and counts and applies each accepted swap to them itself.
 template <int T, class L>
-__global__ void __launch_bounds__(512, 2) mc_large_kernel(const SearchConst c, const McArgs g)
+__global__ void __launch_bounds__(512, 2) mc_large_kernel(const __grid_constant__ SearchConst c, const McArgs g)
 {
     constexpr int S = L::S, NC = S * T * T, NCP = mc_ncount_pad(NC);
+    constexpr int W = SiteHist<T, S, L::kImplicit>::W;
+    using H = SiteHist<T, S, L::kImplicit>;
+    using Record = SwapRecord<W>;
     extern __shared__ __align__(16) uint8_t smem[];
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank(), csize = (int)cluster.num_blocks();
     const int sol = blockIdx.x / csize;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    double2 *tab = reinterpret_cast<double2 *>(smem);
-    SwapRecord *rec = reinterpret_cast<SwapRecord *>(tab + delta_entries(T, S));  // [2][nwarps]
-    int32_t *cnt2 = reinterpret_cast<int32_t *>(rec + 2 * nwarps);                // [2][NCP]
-    SwapRecord *cta_rec = reinterpret_cast<SwapRecord *>(cnt2 + 2 * NCP);         // [2]: this CTA's best
+    const DeltaTab<T, S> tab{reinterpret_cast<float *>(smem)};
+    Record *rec = reinterpret_cast<Record *>(tab.f + DeltaTab<T, S>::kFloats);  // [2][nwarps]
+    Record *cta_rec = rec + 2 * nwarps;                                   // [2]: this CTA's best
+    int32_t *cnt2 = reinterpret_cast<int32_t *>(cta_rec + 2);             // [2][NCP]
 
     const int slot = g.order[sol];
     const uint32_t stream = (g.mc_call << 16) | (uint32_t)sol;
     uint8_t *row = g.occ + (size_t)slot * c.occ_stride;
-    uint4 *hist = g.hist + (size_t)slot * c.num_sites;
+    uint64_t *hist = g.hist + (size_t)slot * c.num_sites * W;
     int32_t *gcnt = g.cnt + (size_t)slot * NC;
     const int n = c.num_sites;
     // this CTA's share of the row and of the tasks
-    const int part = (n + csize - 1) / csize, lo = rank * part, hi = min(n, lo + part);
+    const int part = (n + csize - 1) / csize, row_lo = rank * part, row_hi = min(n, row_lo + part);
     const int qpart = (g.tasks + csize - 1) / csize, qlo = rank * qpart, qhi = min(g.tasks, qlo + qpart);
 
     for (int x = tid; x < NC; x += blockDim.x) cnt2[x] = gcnt[x];
@@ -160,105 +167,82 @@ __global__ void __launch_bounds__(512, 2) mc_large_kernel(const SearchConst c, c
 
     double cur = g.f2[slot];
     int miss = 0, buf = 0;
-    int64_t round = 0, accepts = 0, evals = 0;
+    int64_t round = 0, accepts = 0;
+    uint32_t undrawn = 0;  // this thread's tasks that found no pair
     while (miss < g.depth && round < g.max_rounds) {
-        SwapRecord *rr = rec + (round & 1) * nwarps;
-        SwapRecord &mine = rr[warp];
-        if (lane == 0) {
-            mine.key = kNoSwap;
-            mine.task = 0x7FFFFFFF;
-        }
+        Record *rr = rec + (round & 1) * nwarps;
+        Record &mine = rr[warp];
+        if (lane == 0) mine.lo = mine.hi = kNoSwap;
         __syncwarp();
+        const int32_t *cold = cnt2 + buf * NCP;
         for (int q0 = qlo + warp * 32; q0 < qhi; q0 += blockDim.x) {
             const int q = q0 + lane;
             uint32_t s1 = 0, s2 = 0;
-            uint4 hp = make_uint4(0u, 0u, 0u, 0u), hq = hp;
-            // the species come from the histograms' species words: one L2 round trip per attempt
-            const bool ok = q < qhi && draw_pair_hist(c, stream, (uint32_t)round, (uint32_t)q, hist, s1, s2, hp, hq);
+            Record r;
+            r.p = r.q = HistEntry<W>{};
+            // the species come from the histograms' top bits: one L2 round trip per attempt
+            const bool ok = q < qhi && draw_pair_hist<H>(c, stream, (uint32_t)round, (uint32_t)q, hist, s1, s2, r.p, r.q);
             __syncwarp();
-            uint64_t key = kNoSwap;
-            uint32_t h1[S], h2[S];
-            int a = 0, b = 0;
-            if (ok) {
-                ++evals;
-                a = (int)hp.w / 5;
-                b = (int)hq.w / 5;
-                key = delta_key(score_delta<T, L>(c, g.nbor, g.nbmask, tab, hp, hq, s1, s2, a, b, h1, h2));
-            }
-            uint64_t wk = key;
-            int wq = key != kNoSwap ? q : 0x7FFFFFFF;
-            warp_argmin(wk, wq);
-            if (key != kNoSwap && wq == q && better(wk, wq, mine.key, mine.task)) {
-                SwapRecord r;
-                r.key = wk;
-                r.task = wq;
-                r.s1 = s1;
-                r.s2 = s2;
-                r.ab = a | (b << 8);
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    r.h1[k] = k < S ? h1[k < S ? k : 0] : 0;
-                    r.h2[k] = k < S ? h2[k < S ? k : 0] : 0;
-                }
-                r.stop = 0;
-                r.pad_ = 0;
-                mine = r;
-            }
-            __syncwarp();
+            undrawn += q < qhi && !ok;
+            const int a = hist_species<H>(r.p), b = hist_species<H>(r.q);
+            r.ab = a | (b << 8);
+            float B;
+            const float D = score_delta<T, L>(c, g.nbor, g.nbmask, tab, r.p, r.q, s1, s2, a, b, B);
+            screen_interval(c, tab, ok, D, B, r.lo, r.hi);
+            r.task = q;
+            r.s1 = s1;
+            r.s2 = s2;
+            r.stop = 0;
+            r.pad_ = 0;
+            keep_best<T, L>(c, cold, mine, r, q0 != qlo + warp * 32);
         }
         __syncthreads();
         // this CTA's best record, published for the cluster
         if (warp == 0) {
-            uint64_t xk = lane < nwarps ? rr[lane].key : kNoSwap;
-            int xq = lane < nwarps ? rr[lane].task : 0x7FFFFFFF;
-            const uint64_t own_k = xk;
-            const int own_q = xq;
-            warp_argmin(xk, xq);
-            const int xw = __ffs(__ballot_sync(0xFFFFFFFFu, own_k == xk && own_q == xq)) - 1;
-            if (lane == 0) cta_rec[round & 1] = rr[xw];
+            const int xw = best_record<T, L>(c, cold, lane < nwarps ? rr[lane].lo : kNoSwap,
+                                             lane < nwarps ? rr[lane].hi : kNoSwap, nwarps,
+                                             [rr](int i) -> const Record & { return rr[i]; });
+            if (lane == 0) {
+                if (xw >= 0)
+                    cta_rec[round & 1] = rr[xw];
+                else
+                    cta_rec[round & 1].lo = cta_rec[round & 1].hi = kNoSwap;
+            }
         }
         cluster.sync();
         // every warp reduces the cluster's records
-        uint64_t xk = kNoSwap;
-        int xq = 0x7FFFFFFF;
+        float lo = kNoSwap, hi = kNoSwap;
         if (lane < csize) {
-            const SwapRecord *remote = cluster.map_shared_rank(&cta_rec[round & 1], lane);
-            xk = remote->key;
-            xq = remote->task;
+            const Record *remote = cluster.map_shared_rank(&cta_rec[round & 1], lane);
+            lo = remote->lo;
+            hi = remote->hi;
         }
-        const uint64_t own_k = xk;
-        const int own_q = xq;
-        warp_argmin(xk, xq);
-        if (xk != kNoSwap) {
-            const int xr = __ffs(__ballot_sync(0xFFFFFFFFu, own_k == xk && own_q == xq)) - 1;
-            const SwapRecord w = *cluster.map_shared_rank(&cta_rec[round & 1], xr);
-            const int a = w.ab & 0xFF, b = (w.ab >> 8) & 0xFF;
-            const int32_t *cold = cnt2 + buf * NCP;
+        const int xr = best_record<T, L>(c, cold, lo, hi, csize, [&cluster, cta_rec, round](int i) {
+            return *cluster.map_shared_rank(&cta_rec[round & 1], i);
+        });
+        if (xr >= 0) {
+            const Record w = *cluster.map_shared_rank(&cta_rec[round & 1], xr);
+            const int a = w.ab & 0xFF, b = w.ab >> 8;
             int32_t *cnew = cnt2 + (buf ^ 1) * NCP;
-            const auto after = [cold, &w, a, b](int k, int i, int j) {
-                return cold[(k * T + i) * T + j] + count_change<T>(w, a, b, k, i, j);
-            };
-            const int me = block_rotation(32 * accept_linear_warps<T, S>());
-            for (int x = me; x < NC; x += blockDim.x) cnew[x] = after(x / (T * T), (x / T) % T, x % T);
-            delta_linear<T, S>(c, tab, after);
+            accept_counts<T, L>(tab, w, a, b, cold, cnew);
             if (rank == 0)
-                update_hist<L, true>(c, g.nbor, hist, w.s1, w.s2, a, b,
-                                     block_rotation(32 * (accept_linear_warps<T, S>() + (NC + 31) / 32)));
-            // the cluster's next proposals read the histograms and species words rank 0 updated: rank 0
+                update_hist<T, L, true>(c, g.nbor, hist, w.s1, w.s2, a, b, block_rotation(32 * DeltaTab<T, S>::kWarps));
+            // the cluster's next proposals read the histograms and species bits rank 0 updated: rank 0
             // arrives with release semantics, the others (whose accept work stays in their own shared
-            // memory) relaxed, every thread waits with acquire semantics.  Measured: 4 % per round.
+            // memory, ordered by the block barrier) relaxed, every thread waits with acquire semantics.  Measured: 4 % per round.
+            __syncthreads();  // this CTA's warps read the new counts and table
             if (rank == 0)
-                asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+                __cluster_barrier_arrive();
             else
-                asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+                __cluster_barrier_arrive_relaxed();
+            __cluster_barrier_wait();
+            if (g.trace && rank == 0 && warp == 0) cur = __dadd_rn(cur, exact_delta<T, L>(c, cold, a, b, w.p, w.q));
             buf ^= 1;
-            cur = __dadd_rn(cur, key_delta(xk));
             if (g.trace && rank == 0 && warp == 0 && accepts < g.trace_cap) {
                 if (lane == 0) {
                     AcceptRecord r;
                     r.round = (uint32_t)round;
-                    r.task = (uint32_t)xq;
+                    r.task = (uint32_t)w.task;
                     r.s1 = w.s1;
                     r.s2 = w.s2;
                     r.f2 = cur;
@@ -276,11 +260,17 @@ __global__ void __launch_bounds__(512, 2) mc_large_kernel(const SearchConst c, c
         }
         ++round;
     }
-    cluster.sync();  // rank 0's last species words are visible
-    for (int s = lo + tid; s < hi; s += blockDim.x) row[s] = (uint8_t)(__ldcg(&hist[s].w) / 5u);
+    cluster.sync();  // rank 0's last species bits are visible
+    for (int s = row_lo + tid; s < row_hi; s += blockDim.x) {
+        HistEntry<W> e, same;
+        load_hist_pair<W>(c, hist, (uint32_t)s, (uint32_t)s, e, same);
+        row[s] = (uint8_t)hist_species<H>(e);
+    }
     if (rank == 0)
         for (int x = tid; x < NC; x += blockDim.x) gcnt[x] = cnt2[buf * NCP + x];
-    unsigned long long ev = (unsigned long long)evals;
+    const int share = max(0, qhi - qlo);  // this CTA's tasks
+    const int64_t scored = (int64_t)(tid < share ? (share - 1 - tid) / (int)blockDim.x + 1 : 0) * round;
+    unsigned long long ev = (unsigned long long)(scored - undrawn);
 #pragma unroll
     for (int o = 16; o; o >>= 1) ev += __shfl_xor_sync(0xFFFFFFFFu, ev, o);
     if (lane == 0 && ev) atomicAdd(&g.stats[1], ev);

@@ -8,10 +8,10 @@
 //   cnt    int32 [slots][S][T][T]      pair counts that travel with their slot
 //   f2     double [slots]              squared weighted SRO error
 //   order  int32 [2P]                  slot ids: current population, then the new one
-// In shared memory a slot's occupancy is held as 5*species (the shift of its
-// 5-bit histogram field), plus the sentinel byte 0 at index N.
+// In shared memory a slot's occupancy has the sentinel byte 0 at index N.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 #include <utility>
 
 #include "hea_device.cuh"
@@ -31,7 +31,7 @@ struct LatticeConst {
     int32_t L;                   // cube edge in cells; 0: the structure has a neighbour table
     int32_t nb;                  // basis sites per cell (4 FCC, 2 BCC)
     int32_t zsize[3], zoff[3];   // shell sizes and offsets in the concatenated neighbour list
-    double inv_L, inv_LL;        // 1 / L and 1 / L^2, rounded (lattice_cell)
+    uint32_t mul_L, mul_LL;      // floor(2^32 / L) and floor(2^32 / L^2) (lattice_cell)
     int32_t kind;                // kLatFccRef, kLatFccTrue3 or kLatBcc
     int32_t pad_;
 };
@@ -46,11 +46,14 @@ struct SearchConst {
     int32_t pad[kMaxShells];      // sentinel entries in the segment
     int32_t prefix[kMaxTypes + 1];  // species prefix sums
     int32_t num_sites, row4, occ_stride, num_types, num_shells, feistel_h;
-    uint32_t reject_below, key0, key1;
+    uint32_t key0, key1;
     uint32_t draw16;    // 1: 16-bit draws, four attempts per Philox call (use_draw16)
-    uint32_t reject16;  // 2^16 mod N
-    uint32_t hist_stream;  // 1: site histograms read with streaming (evict-first) loads (load_hist)
-    uint32_t pad_;
+    uint32_t reject;    // draws whose product has a lower remainder are rejected: 2^32 mod N, or (2^16 mod N) << 16
+    uint32_t hist_stream;  // 1: site histograms read with streaming (evict-first) loads (load_hist_pair)
+    float screen_floor;    // 0; 3e38 when FP32's range does not hold the structure: every D is then exact
+    double screen_scale;   // power of two that brings the largest Q to about 1 in the FP32 table
+    float screen_sw[kMaxShells + 1];           // sqrt(w * screen_scale), rounded up
+    float kappa[kMaxTypes * kMaxTypes];        // max(1, n_t / n_i) at [i][t], rounded up
     LatticeConst lat;   // lat.L > 0: neighbours from lattice arithmetic (nbor unused)
 };
 
@@ -133,12 +136,11 @@ __host__ __device__ constexpr LatDescTable make_lat_desc_table()
 }
 __device__ const LatDescTable kLatDesc = make_lat_desc_table();
 
-// floor(n / d) for 0 <= n < 2^31, d <= 2^20, from inv = 1/d rounded: n * inv is
-// within 2^-21 of n / d, so the truncation is the quotient or one less, and
-// one correction makes it exact.
-__device__ __forceinline__ int div_by(int n, int d, double inv)
+// floor(n / d) for 0 <= n < 2^31, d >= 2, from m = floor(2^32 / d): n m / 2^32
+// is within n / 2^32 < 1 of n / d, so its floor is the quotient or one less.
+__device__ __forceinline__ int div_by(int n, int d, uint32_t m)
 {
-    int q = __double2int_rz(__dmul_rn((double)n, inv));
+    int q = (int)__umulhi((uint32_t)n, m);
     q += (n - q * d) >= d;
     return q;
 }
@@ -150,7 +152,7 @@ struct LatticeCell {
 __device__ __forceinline__ LatticeCell lattice_cell(const LatticeConst &lc, int s)
 {
     const int cell = s >> (lc.nb == 4 ? 2 : 1), LL = lc.L * lc.L;  // nb is 2 or 4
-    const int x = div_by(cell, LL, lc.inv_LL), r = cell - x * LL, y = div_by(r, lc.L, lc.inv_L);
+    const int x = div_by(cell, LL, lc.mul_LL), r = cell - x * LL, y = div_by(r, lc.L, lc.mul_L);
     return LatticeCell{s & (lc.nb - 1), x, y, r - y * lc.L};
 }
 
@@ -334,8 +336,8 @@ struct McArgs {
     uint8_t *occ;
     int32_t *cnt;
     double *f2;
-    uint4 *hist;              // [slots][N] site histograms (see block_recount)
-    const uint32_t *nbmask;   // neighbour-offset bitmap (see score_swap_hist)
+    uint64_t *hist;           // [slots][N] site histograms (SiteHist)
+    const uint32_t *nbmask;   // neighbour-offset bitmap (score_delta)
     const int32_t *order;  // slots searched by this launch, one CTA each
     uint32_t mc_call;
     int32_t tasks, depth;
@@ -354,7 +356,7 @@ struct GenArgs {
     uint8_t *occ;
     int32_t *cnt;
     double *f2;
-    uint4 *hist;  // [slots][N] site histograms written by the recount (nullptr: none)
+    uint64_t *hist;  // [slots][N] site histograms written by the recount (nullptr: none)
     const int32_t *order;
     uint32_t generation;
     int32_t generate;  // 1: draw a new occupancy; 0: recount the stored one
@@ -404,12 +406,8 @@ __device__ __forceinline__ double fitness_of_counts(const SearchConst &c, const 
 //     L_t = -2 (G_at - G_bt),   G_it = R_it (d_it + d_ti),
 //     Q_t = 2 (R_at^2 + R_bt^2) for t != a, b,   Q_a = 4 R_aa^2,   Q_b = 4 R_bb^2,
 //     Cq  = 2 R_ab^2,
-// and f2 changes by D = sum_k w_k (that).  Each search keeps, per shell k and
-// ordered pair (a, b), the row {w L_t, w Q_t} (t < T), {w Cq, 0} in shared
-// memory (the delta table; Q and Cq depend on the structure only, L on the
-// counts and is rebuilt after every accepted swap) and scores a proposal by D
-// alone: O(T) terms per shell instead of the O(T^2) of a full fitness.
-// Fixed operation order (restated by the CPU oracle):
+// and f2 changes by D = sum_k w_k (that): O(T) terms per shell instead of the
+// O(T^2) of a full fitness.  Fixed operation order (restated by the CPU oracle):
 //     Q   = w * (2 * (R_at * R_at + R_bt * R_bt)),  Q_a = w * (4 * (R_aa * R_aa)),
 //     Cq  = w * (2 * (R_ab * R_ab)),
 //     d_it = fma(-C, R_it, E_it),  G_it = R_it * (d_it + d_ti),  L = (-2 * w) * (G_at - G_bt),
@@ -417,147 +415,572 @@ __device__ __forceinline__ double fitness_of_counts(const SearchConst &c, const 
 // A round's best proposal (lowest D, lowest task on ties) is accepted iff D < 0;
 // the search's running f2 adds D, and the f2 a search stores at its end is
 // recomputed from the counts (fitness_of_counts).
+//
+// Which proposal wins is all a round needs of the D's, so they are screened:
+// every proposal gets an FP32 value of D and a bound e on its distance from D
+// (score_delta), and the FP64 D above is computed (exact_delta) only for those
+// whose intervals [D32 - e, D32 + e] leave the winner or its sign open --
+// almost always none.  The winner is the same as if all D were compared.
+//
+// The FP32 table (DeltaTab, shared memory) holds, scaled by a power of two,
+// per shell k and ordered pair (a, b) the row of L_t (from the counts, rebuilt
+// after every accepted swap) and Q_t, and Cq apart.
+//
+// The bound: with delta = 2^-24, g_xt = 2 w |G_xt| and A = sum |u_t| (g_at + g_bt),
+// the L's are differences of twice rounded g's and all sums together round at most 20
+// times, so |D32 - D| <= 24 delta (A + B), B = sum u_t^2 Q_t + sum (u_a - u_b)^2 Cq
+// (all positive).  By Cauchy-Schwarz A^2 <= B sum_kt (g_at + g_bt)^2 / Q_t, and
+// every (g_at + g_bt)^2 / Q_t is at most 4 max_i w (kappa_it (d_it + d_ti))^2 with
+// kappa_it = max(1, n_t / n_i) (it matters for t = a or b, whose Q holds R_tt
+// alone).  So e = 32 delta (B + sqrt(B) z), z^2 = 4 S T max_kit w (kappa_it (d_it + d_ti))^2,
+// kept with the table; 32 leaves room for the roundings of e itself and of D.
+// It holds while the table's values stay in FP32's range, which the host
+// checks (SearchConst::screen_floor).
 // ---------------------------------------------------------------------------
-__host__ __device__ constexpr int delta_row(int T) { return (T + 1) | 1; }  // odd: lanes' rows spread over the banks
-__host__ __device__ constexpr int delta_entries(int T, int S) { return S * T * T * delta_row(T); }  // double2 entries
+constexpr float kNoSwap = 3.0e38f;  // lo and hi of no proposal, or of one that does not improve
+constexpr float kScreenEps = 32.0f / 16777216.0f;
 
-// Structure constants of the table: w Q_t in .y of entries t < T, w Cq in .x
-// of entry T, for every (k, a, b), a != b.  Block-cooperative, no barrier.
+// Layout of the FP32 table, in floats: rows of (k, a, b), within a row species
+// t < 2 kPairs in groups {L_t, L_t+1, Q_t, Q_t+1} (one 16-byte load, packed FMAs),
+// then {L, Q} of each species left (one or two); Cq [S][T][T]; the coefficients
+// of u_a - u_b in the stored u_t, [T][T][kSaRow]; z as found by each warp that
+// rebuilds L; the exact D of the accepted swap; and per lane that rebuilds L its
+// constants (delta_linear).  Rows are an odd number of 16-byte units apart, which
+// spreads lanes' random rows over the banks.
 template <int T, int S>
-__device__ void delta_consts(const SearchConst &c, double2 *tab)
-{
-    constexpr int R = delta_row(T);
-    for (int e = threadIdx.x; e < S * T * T * R; e += blockDim.x) {
-        const int t = e % R, ab = (e / R) % (T * T), k = e / (R * T * T);
-        const int a = ab / T, b = ab % T;
-        if (a == b || t > T) continue;
-        const double *Rk = c.R + k * T * T;
-        const double w = c.w[k];
-        if (t == T) {
-            tab[e].x = __dmul_rn(w, __dmul_rn(2.0, __dmul_rn(Rk[a * T + b], Rk[a * T + b])));
-        } else if (t == a || t == b) {
-            tab[e].y = __dmul_rn(w, __dmul_rn(4.0, __dmul_rn(Rk[t * T + t], Rk[t * T + t])));
-        } else {
-            const double p = __dmul_rn(Rk[a * T + t], Rk[a * T + t]), q = __dmul_rn(Rk[b * T + t], Rk[b * T + t]);
-            tab[e].y = __dmul_rn(w, __dmul_rn(2.0, __dadd_rn(p, q)));
-        }
+struct DeltaTab {
+    static constexpr int kPairs = (T - 1) / 2, kRest = T - 2 * kPairs, kRow = T == 2 ? 4 : 12, kRows = S * T * T;
+    static constexpr int kGroups = 32 / T, kWarps = (S * T + kGroups - 1) / kGroups;  // warps that rebuild L
+    static constexpr int kSaRow = T == 6 ? 8 : 4;
+    static constexpr int kCq = kRows * kRow, kSa = (kCq + kRows + 3) & ~3, kZ = kSa + T * T * kSaRow,
+                         kAccepted = kZ + 4, kLanes = kAccepted + 4, kFloats = kLanes + kWarps * 32 * 6;
+    static_assert(kWarps <= 4, "one z slot per warp");
+    static constexpr float kZScale = S * T <= 4 ? 4.0f : S * T <= 9 ? 6.0f : S * T <= 16 ? 8.0f : 8.5f;  // >= sqrt(4 S T)
+    float *f;
+    __host__ __device__ static constexpr int lin(int t)
+    {
+        return t < 2 * kPairs ? 4 * (t / 2) + (t & 1) : 4 * kPairs + 2 * (t - 2 * kPairs);
     }
+    __host__ __device__ static constexpr int quad(int t) { return lin(t) + (t < 2 * kPairs ? 2 : 1); }
+    __device__ __forceinline__ float *row(int k, int a, int b) const { return f + ((k * T + a) * T + b) * kRow; }
+    __device__ __forceinline__ double *accepted() const { return reinterpret_cast<double *>(f + kAccepted); }
+    // lane constants of entry i = 32 w + lane: 2 R_xt and E_xt + E_tx; -2 w R_xt and kappa_xt sqrt(w), scaled
+    __device__ __forceinline__ double *lane_r2() const { return reinterpret_cast<double *>(f + kLanes); }
+    __device__ __forceinline__ double *lane_e() const { return lane_r2() + kWarps * 32; }
+    __device__ __forceinline__ float *lane_g() const { return f + kLanes + kWarps * 32 * 4; }
+    __device__ __forceinline__ float *lane_z() const { return lane_g() + kWarps * 32; }
+};
+template <int T>
+__host__ __device__ constexpr size_t delta_floats(int S)
+{
+    return S == 1 ? DeltaTab<T, 1>::kFloats : S == 2 ? DeltaTab<T, 2>::kFloats : DeltaTab<T, 3>::kFloats;
+}
+__host__ __device__ constexpr size_t delta_bytes(int T, int S)
+{
+    return sizeof(float) * (T == 2   ? delta_floats<2>(S)
+                            : T == 3 ? delta_floats<3>(S)
+                            : T == 4 ? delta_floats<4>(S)
+                            : T == 5 ? delta_floats<5>(S)
+                                     : delta_floats<6>(S));
 }
 
-// The count-dependent half of the table: w L_t in .x of entries t < T, from
-// the counts count_of(k, i, j) (symmetric in i, j).  Groups of T lanes of a
-// warp hold G_xt for x = 0..T-1 of one (shell, t); each lane takes the others'
-// G by shuffle and writes its row x against every y != x.  Warps call it
-// convergently (full-mask shuffles); no barrier inside.
-template <int T, int S, class CountOf>
-__device__ __forceinline__ void delta_linear(const SearchConst &c, double2 *tab, CountOf count_of)
+// Q_t of the pair (a, b) in one shell's R, and Cq.
+template <int T>
+__device__ __forceinline__ double delta_quad(const double *Rk, double w, int a, int b, int t)
 {
-    constexpr int R = delta_row(T), kGroups = 32 / T, kWarps = (S * T + kGroups - 1) / kGroups;
+    if (t == a || t == b) return __dmul_rn(w, __dmul_rn(4.0, __dmul_rn(Rk[t * T + t], Rk[t * T + t])));
+    const double p = __dmul_rn(Rk[a * T + t], Rk[a * T + t]), q = __dmul_rn(Rk[b * T + t], Rk[b * T + t]);
+    return __dmul_rn(w, __dmul_rn(2.0, __dadd_rn(p, q)));
+}
+template <int T>
+__device__ __forceinline__ double delta_cross(const double *Rk, double w, int a, int b)
+{
+    return __dmul_rn(w, __dmul_rn(2.0, __dmul_rn(Rk[a * T + b], Rk[a * T + b])));
+}
+
+// Structure constants of the table: Q and Cq of every (k, a, b), a != b, the
+// coefficients of u_a - u_b, the lanes' constants, and the z slots no warp writes.
+// Block-cooperative, no barrier.
+template <int T, int S>
+__device__ void delta_consts(const SearchConst &c, const DeltaTab<T, S> tab)
+{
+    using Tab = DeltaTab<T, S>;
+    const double scale = c.screen_scale;  // 0: beyond FP32's range, the table is all zero
+    for (int e = threadIdx.x; e < S * T * T * T; e += blockDim.x) {
+        const int t = e % T, ab = (e / T) % (T * T), k = e / (T * T * T), a = ab / T, b = ab % T;
+        if (a == b) continue;
+        const double *R = c.R + k * T * T;
+        tab.row(k, a, b)[Tab::quad(t)] = scale > 0.0 ? (float)(scale * delta_quad<T>(R, c.w[k], a, b, t)) : 0.0f;
+        if (t == 0)
+            tab.f[Tab::kCq + k * T * T + ab] = scale > 0.0 ? (float)(scale * delta_cross<T>(R, c.w[k], a, b)) : 0.0f;
+        // u of the last species is minus the sum of the others
+        if (k == 0 && t < T - 1)
+            tab.f[Tab::kSa + ab * Tab::kSaRow + t] =
+                (float)((t == a) - (t == b) - (T - 1 == a) + (T - 1 == b));
+    }
+    for (int i = threadIdx.x; i < 32 * Tab::kWarps; i += blockDim.x) {
+        const int x = (i & 31) % T, grp = (i & 31) / T, g = (i >> 5) * Tab::kGroups + grp;
+        const bool on = grp < Tab::kGroups && g < S * T;
+        const int k = on ? g / T : 0, t = on ? g % T : 0, xt = (k * T + x) * T + t, tx = (k * T + t) * T + x;
+        tab.lane_r2()[i] = scale > 0.0 ? 2.0 * c.R[xt] : 0.0;
+        tab.lane_e()[i] = scale > 0.0 ? c.E[xt] + c.E[tx] : 0.0;
+        tab.lane_g()[i] = scale > 0.0 ? (float)(-2.0 * scale * c.w[k] * c.R[xt]) : 0.0f;
+        tab.lane_z()[i] = on && scale > 0.0 ? c.kappa[x * T + t] * c.screen_sw[k] : 0.0f;
+    }
+    if (threadIdx.x >= Tab::kWarps && threadIdx.x < 4) tab.f[Tab::kZ + threadIdx.x] = 0.0f;
+}
+
+// The count-dependent part of the table: L of every row, from the counts
+// count_of(k, i, j) (symmetric in i, j), and z; with `cnew`, also stores the
+// counts there.  Groups of T lanes of a warp hold G_xt for x = 0..T-1 of one
+// (shell, t) -- all (k, x, t) once; each lane takes the others' G by shuffle and
+// writes its row x against every y != x.  Warps call it convergently (full-mask
+// shuffles, also in count_of); no barrier inside.
+//
+// It is the longest chain of an accepted round, so the lanes' constants lie in
+// shared memory, one conflict-free load each (as indexed loads from the
+// kernel's parameters they replayed once per lane).
+template <int T, int S, class CountOf>
+__device__ __forceinline__ void delta_linear(const DeltaTab<T, S> tab, int32_t *cnew, CountOf count_of)
+{
+    using Tab = DeltaTab<T, S>;
     const int lane = threadIdx.x & 31, x = lane % T, grp = lane / T;
-    for (int w = threadIdx.x >> 5; w < kWarps; w += blockDim.x >> 5) {
-        const int g = w * kGroups + grp;  // shell k = g / T, column t = g % T
-        const bool on = grp < kGroups && g < S * T;
-        const int k = on ? g / T : 0, t = on ? g % T : 0;
-        const int xt = (k * T + x) * T + t, tx = (k * T + t) * T + x;
-        double G = 0.0, m2w = 0.0;
-        if (on) {
-            const double C = (double)count_of(k, x, t);
-            const double dxt = __fma_rn(-C, c.R[xt], c.E[xt]);
-            const double dtx = __fma_rn(-C, c.R[xt], c.E[tx]);
-            G = __dmul_rn(c.R[xt], __dadd_rn(dxt, dtx));
-            m2w = __dmul_rn(-2.0, c.w[k]);
-        }
+    for (int w = threadIdx.x >> 5; w < Tab::kWarps; w += blockDim.x >> 5) {
+        const int g = w * Tab::kGroups + grp, i = 32 * w + lane;  // shell k = g / T, column t = g % T
+        const bool on = grp < Tab::kGroups && g < S * T;
+        const int k = on ? g / T : 0, t = on ? g - k * T : 0;
+        const int C = count_of(k, x, t);
+        if (cnew && on) cnew[(k * T + x) * T + t] = C;
+        const float dd = (float)__fma_rn(-(double)C, tab.lane_r2()[i], tab.lane_e()[i]);
+        const float G = dd * tab.lane_g()[i], r = dd * tab.lane_z()[i];
+        float *row = tab.row(k, x, 0) + Tab::lin(t);
 #pragma unroll
         for (int y = 0; y < T; ++y) {
-            const double Gy = __shfl_sync(0xFFFFFFFFu, G, lane - x + y);
-            if (on && y != x) tab[((k * T + x) * T + y) * R + t].x = __dmul_rn(m2w, __dsub_rn(G, Gy));
+            const float Gy = __shfl_sync(0xFFFFFFFFu, G, lane - x + y);
+            if (on && y != x) row[y * Tab::kRow] = G - Gy;
         }
+        const float rmax = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(fabsf(r))));
+        if (lane == 0) tab.f[Tab::kZ + w] = rmax * Tab::kZScale;
     }
 }
 
-__device__ __forceinline__ int field5(uint32_t h, int shift) { return (int)((h >> shift) & 31u); }
+// ---------------------------------------------------------------------------
+// Site histograms: per slot and site, how many neighbours of each species the
+// site has in each shell.  A shell's counts sum to its size, so the last
+// species is left out (a difference of two sites' counts of it is minus the
+// sum of the others'), and one 64-bit word holds a site: T - 1 fields of 5
+// bits per shell (Z <= 28 < 32), shells one after the other, and the site's own
+// species in the top 3 bits.  Only six species in three shells need more than
+// 64 bits that way: lattice structures then use the 4, 3 and 5 bits that
+// their shells of at most 12, 6 and 24 neighbours take, tables of any other
+// shells a second word (shell 2 and the species).
+//
+// Why one word: the two entries of a proposal are random loads, and what they
+// cost is set by how much of the population's histograms L2 holds and, beyond
+// it, by DRAM's random-access rate.  Measured on B200 from a 4 GiB buffer:
+// 4.8e10 random 8-byte loads/s against 2.4e10 (3.2e10 evict-first) 16-byte ones.
+// ---------------------------------------------------------------------------
+template <int T, int S, bool kImplicit>
+struct SiteHist {
+    static constexpr bool kWide = T == 6 && S == 3 && !kImplicit;
+    static constexpr bool kTight = T == 6 && S == 3 && kImplicit;
+    static constexpr int W = kWide ? 2 : 1;  // 64-bit words per site
+    static constexpr int kHalves = 2 * W;    // 32-bit words
+    // field (k, t), t < T - 1: its 32-bit word, its place among the word's fields, first bit, width.
+    // Uniform: six 5-bit fields per 32-bit word.  Tight: shell 2 then two fields of shell 1 in the
+    // low word, shell 0 then the other three of shell 1 in the high word.  Wide: a shell per word.
+    __host__ __device__ static constexpr int half(int k, int t)
+    {
+        return kWide ? k : kTight ? (k == 0 ? 1 : k == 2 ? 0 : t < 2 ? 0 : 1) : (k * (T - 1) + t) / 6;
+    }
+    __host__ __device__ static constexpr int place(int k, int t)
+    {
+        return kWide ? t : kTight ? (k != 1 ? t : t < 2 ? 5 + t : 3 + t) : (k * (T - 1) + t) % 6;
+    }
+    __host__ __device__ static constexpr int width(int k) { return kTight ? (k == 0 ? 4 : k == 1 ? 3 : 5) : 5; }
+    __host__ __device__ static constexpr int bit(int k, int t)
+    {
+        return kTight ? (k == 0 ? 4 * t : k == 2 ? 5 * t : t < 2 ? 25 + 3 * t : 14 + 3 * t) : 5 * place(k, t);
+    }
+    __host__ __device__ static constexpr int word(int k, int t) { return half(k, t) / 2; }
+    __host__ __device__ static constexpr int shift(int k, int t) { return 32 * (half(k, t) & 1) + bit(k, t); }
+    // Fields of 32-bit word h at even (odd) places: their mask, and one above each field's top bit
+    // (free in that mask), so that differences of all of them take one subtraction.
+    __host__ __device__ static constexpr uint32_t fields(int h, int parity)
+    {
+        uint32_t m = 0;
+        for (int k = 0; k < S; ++k)
+            for (int t = 0; t < T - 1; ++t)
+                if (half(k, t) == h && (place(k, t) & 1) == parity) m |= ((1u << width(k)) - 1u) << bit(k, t);
+        return m;
+    }
+    __host__ __device__ static constexpr uint32_t guards(int h, int parity)
+    {
+        uint32_t m = 0;
+        for (int k = 0; k < S; ++k)
+            for (int t = 0; t < T - 1; ++t)
+                if (half(k, t) == h && (place(k, t) & 1) == parity) m |= 1u << (bit(k, t) + width(k));
+        return m;
+    }
+};
+// Words per site; the host sizes the histogram buffers with it.
+__host__ __device__ constexpr int hist_words(int T, int S, bool implicit) { return T == 6 && S == 3 && !implicit ? 2 : 1; }
+
+template <int W>
+struct HistEntry {
+    uint64_t w[W];
+    __device__ __forceinline__ uint32_t half(int h) const { return (uint32_t)(w[h / 2] >> (32 * (h & 1))); }
+};
+
+template <class H>
+__device__ __forceinline__ int hist_field(const HistEntry<H::W> &e, int k, int t)  // t < T - 1
+{
+    return (int)((uint32_t)(e.w[H::word(k, t)] >> H::shift(k, t)) & ((1u << H::width(k)) - 1u));
+}
+template <class H, int T>
+__device__ __forceinline__ uint64_t hist_unit(int k, int t)  // one neighbour of species t in shell k
+{
+    return t < T - 1 ? 1ull << H::shift(k, t) : 0ull;
+}
+// The site's own species: in six-species three-shell structures the top 3 bits;
+// else bits 62 and 63, with bit 31 above them (the uniform fields leave bits 30, 31, 62 and 63 free).
+template <class H>
+__device__ __forceinline__ int hist_species(const HistEntry<H::W> &e)
+{
+    const uint64_t w = e.w[H::W - 1];
+    if constexpr (H::kWide || H::kTight) return (int)(w >> 61);
+    return (int)(w >> 62) | (int)(((uint32_t)w >> 31) << 2);
+}
+template <class H>
+__device__ __forceinline__ uint64_t hist_species_bits(int a)
+{
+    if constexpr (H::kWide || H::kTight) return (uint64_t)a << 61;
+    return ((uint64_t)(a & 3) << 62) | ((uint64_t)(a >> 2) << 31);
+}
+
+// Two sites' entries, through L2.  Structures whose histograms are far larger
+// than L2 (SearchConst::hist_stream, set by the host) read them evict-first, so
+// that random lines from DRAM do not push out those that are read again.
+template <int W>
+__device__ __forceinline__ void load_hist_pair(const SearchConst &c, const uint64_t *hist, uint32_t s1, uint32_t s2,
+                                               HistEntry<W> &p, HistEntry<W> &q)
+{
+    if constexpr (W == 1) {
+        const unsigned long long *h = reinterpret_cast<const unsigned long long *>(hist);
+        if (c.hist_stream) {
+            p.w[0] = __ldcs(h + s1);
+            q.w[0] = __ldcs(h + s2);
+        } else {
+            p.w[0] = __ldcg(h + s1);
+            q.w[0] = __ldcg(h + s2);
+        }
+    } else {
+        const ulonglong2 *h = reinterpret_cast<const ulonglong2 *>(hist);
+        const ulonglong2 x = c.hist_stream ? __ldcs(h + s1) : __ldcg(h + s1);
+        const ulonglong2 y = c.hist_stream ? __ldcs(h + s2) : __ldcg(h + s2);
+        p.w[0] = x.x;
+        p.w[1] = x.y;
+        q.w[0] = y.x;
+        q.w[1] = y.y;
+    }
+}
 
 __device__ __forceinline__ int count4(const int4 x, uint32_t v)
 {
     return ((uint32_t)x.x == v) + ((uint32_t)x.y == v) + ((uint32_t)x.z == v) + ((uint32_t)x.w == v);
 }
 
-// D of one proposal: s1 (species a, site histograms p), s2 (b, q).  On return
-// h1, h2 are the shell histograms with m folded in -- h1_k + (m << 5a), h2_k +
-// (m << 5b) -- so that u_t = field_t(h2_k) - field_t(h1_k); the fields stay
-// below 32 (n1_a + m <= Z_k because s1's list holds s2, of species b, m times;
-// likewise for h2).  nbmask has bit (n - s + N - 1) set for every table entry n
-// of every site s: a clear bit for s2 - s1 proves m = 0 in every shell, a set
-// bit sends the lane to count s2 in s1's row.
-template <int T, class L>
-__device__ __forceinline__ double score_delta(const SearchConst &c, const int4 *__restrict__ nbor,
-                                              const uint32_t *__restrict__ nbmask, const double2 *tab, const uint4 p,
-                                              const uint4 q, uint32_t s1, uint32_t s2, int a, int b,
-                                              uint32_t (&h1)[L::S], uint32_t (&h2)[L::S])
+// d = a * b + c on two floats at once (one instruction on sm_100).
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c)
 {
-    constexpr int S = L::S, R = delta_row(T);
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(d)
+        : "l"(*reinterpret_cast<uint64_t *>(&a)), "l"(*reinterpret_cast<uint64_t *>(&b)),
+          "l"(*reinterpret_cast<uint64_t *>(&c)));
+    return *reinterpret_cast<float2 *>(&d);
+}
+__device__ __forceinline__ float2 fmul2(float2 a, float2 b)
+{
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;"
+        : "=l"(d)
+        : "l"(*reinterpret_cast<uint64_t *>(&a)), "l"(*reinterpret_cast<uint64_t *>(&b)));
+    return *reinterpret_cast<float2 *>(&d);
+}
+__device__ __forceinline__ float2 fadd2(float2 a, float2 b)
+{
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;"
+        : "=l"(d)
+        : "l"(*reinterpret_cast<uint64_t *>(&a)), "l"(*reinterpret_cast<uint64_t *>(&b)));
+    return *reinterpret_cast<float2 *>(&d);
+}
+__device__ __forceinline__ float sqrt_approx(float x)
+{
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// u_t = field_t(q) - field_t(p) of every stored species and shell as floats:
+// all differences of a word's even or odd places at once, each biased by its
+// guard bit; then each field, where it stands, becomes the low mantissa bits of
+// a power of two whose last place is the field's first bit.
+template <class H, int T, int S>
+__device__ __forceinline__ void hist_diff(const HistEntry<H::W> &p, const HistEntry<H::W> &q, float (&u)[S][T])
+{
+    uint32_t d[H::kHalves][2];
+#pragma unroll
+    for (int h = 0; h < H::kHalves; ++h)
+#pragma unroll
+        for (int y = 0; y < 2; ++y)
+            d[h][y] = (q.half(h) & H::fields(h, y)) - (p.half(h) & H::fields(h, y)) + H::guards(h, y);
+#pragma unroll
+    for (int k = 0; k < S; ++k)
+#pragma unroll
+        for (int t = 0; t < T - 1; ++t) {
+            const uint32_t x = d[H::half(k, t)][H::place(k, t) & 1], field = (2u << H::width(k)) - 1u;
+            const int bit = H::bit(k, t), at = bit + H::width(k) + 1 <= 23 ? bit : bit - 20;  // or 20 places down
+            u[k][t] = __uint_as_float(((bit == at ? x : x >> 20) & (field << at)) | ((uint32_t)(150 - at) << 23)) -
+                      ((float)(1u << (23 - at)) + (float)(1u << H::width(k)));
+        }
+}
+
+// The FP32 value of one proposal's (scaled) D, and B of its bound: s1 (species
+// a, site histograms p), s2 (b, q).  On return p and q have m folded in -- m
+// added to field a of p's shell k and to field b of q's -- so that u_t =
+// field_t(q) - field_t(p), and u of the last species is minus the sum of the
+// others (both totals are Z_k + m); the fields keep their width (n1_a + m <= Z_k
+// because s1's list holds s2, of species b, m times; likewise for q).  nbmask has
+// bit (n - s + N - 1) set for every table entry n of every site s: a clear bit
+// for s2 - s1 proves m = 0 in every shell, a set bit sends the lane to count s2
+// in s1's row.
+//
+// What bounds it: shared-memory wavefronts (lanes read random rows) and issue
+// slots.  Per shell of five species: three 16-byte row loads instead of five of
+// the FP64 form, packed FMAs, no int-to-double conversions.
+template <int T, class L, int W>
+__device__ __forceinline__ float score_delta(const SearchConst &c, const int4 *__restrict__ nbor,
+                                             const uint32_t *__restrict__ nbmask, const DeltaTab<T, L::S> tab,
+                                             HistEntry<W> &p, HistEntry<W> &q, uint32_t s1, uint32_t s2, int a, int b,
+                                             float &B)
+{
+    constexpr int S = L::S;
+    using H = SiteHist<T, S, L::kImplicit>;
+    using Tab = DeltaTab<T, S>;
     const uint32_t d = s2 - s1 + (uint32_t)c.num_sites - 1u;
     const bool near = (__ldg(nbmask + (d >> 5)) >> (d & 31u)) & 1u;
-    const uint32_t pv[3] = {p.x, p.y, p.z}, qv[3] = {q.x, q.y, q.z};
-#pragma unroll
-    for (int k = 0; k < S; ++k) {
-        h1[k] = pv[k];
-        h2[k] = qv[k];
-    }
-    const int a5 = 5 * a, b5 = 5 * b;
     if (near) {
+        uint32_t m[S];
         if constexpr (L::kImplicit) {
-            uint32_t m[S];
             lattice_multiplicity<S>(c.lat, (int)s1, (int)s2, m);
-#pragma unroll
-            for (int k = 0; k < S; ++k) {
-                h1[k] += m[k] << a5;
-                h2[k] += m[k] << b5;
-            }
         } else {
             const int row4 = L::kRuntime ? c.row4 : L::kRow4;
             const int4 *r1 = nbor + (size_t)s1 * row4;
 #pragma unroll
             for (int k = 0; k < S; ++k) {
                 const int o = L::kRuntime ? c.off4[k] : L::off(k), n = L::kRuntime ? c.chunks[k] : L::chunks(k);
-                uint32_t m = 0;
-                for (int ch = 0; ch < n; ++ch) m += count4(__ldg(r1 + o + ch), s2);
-                h1[k] += m << a5;
-                h2[k] += m << b5;
+                m[k] = 0;
+                for (int ch = 0; ch < n; ++ch) m[k] += count4(__ldg(r1 + o + ch), s2);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < S; ++k) {
+#pragma unroll
+            for (int x = 0; x < W; ++x) {
+                p.w[x] += (W == 1 || H::word(k, 0) == x) ? m[k] * hist_unit<H, T>(k, a) : 0ull;
+                q.w[x] += (W == 1 || H::word(k, 0) == x) ? m[k] * hist_unit<H, T>(k, b) : 0ull;
             }
         }
     }
-    const double2 *row = tab + (a * T + b) * R;
+    float u[S][T];
+    hist_diff<H, T, S>(p, q, u);
+    const float *row = tab.row(0, a, b), *cq = tab.f + Tab::kCq + a * T + b;
+    const float4 s4 = *reinterpret_cast<const float4 *>(tab.f + Tab::kSa + (a * T + b) * Tab::kSaRow);
+    const float sa[5] = {s4.x, s4.y, s4.z, s4.w, T == 6 ? tab.f[Tab::kSa + (a * T + b) * Tab::kSaRow + 4] : 0.0f};
+    float2 lin2 = make_float2(0.0f, 0.0f), quad2 = lin2;
+    float lin = 0.0f, quad = 0.0f;
+#pragma unroll
+    for (int k = 0; k < S; ++k) {
+        const float *r = row + k * T * T * Tab::kRow;
+        float2 sum2 = make_float2(0.0f, 0.0f), v2 = sum2;  // of the stored u; of sa u: v = u_a - u_b
+#pragma unroll
+        for (int g = 0; g < Tab::kPairs; ++g) {
+            const float4 x = *reinterpret_cast<const float4 *>(r + 4 * g);
+            const float2 uu = make_float2(u[k][2 * g], u[k][2 * g + 1]), ss = make_float2(sa[2 * g], sa[2 * g + 1]);
+            lin2 = ffma2(uu, make_float2(x.x, x.y), lin2);
+            quad2 = ffma2(fmul2(uu, uu), make_float2(x.z, x.w), quad2);
+            sum2 = g ? fadd2(sum2, uu) : uu;
+            v2 = g ? ffma2(uu, ss, v2) : fmul2(uu, ss);
+        }
+        float sum = sum2.x + sum2.y, v = v2.x + v2.y;
+        if constexpr (Tab::kRest == 2) {
+            sum += u[k][T - 2];
+            v = fmaf(u[k][T - 2], sa[T - 2], v);
+        }
+        u[k][T - 1] = -sum;
+        if constexpr (Tab::kRest == 2) {
+            const float4 x = *reinterpret_cast<const float4 *>(r + 4 * Tab::kPairs);
+            lin = fmaf(u[k][T - 2], x.x, lin);
+            quad = fmaf(u[k][T - 2] * u[k][T - 2], x.y, quad);
+            lin = fmaf(u[k][T - 1], x.z, lin);
+            quad = fmaf(u[k][T - 1] * u[k][T - 1], x.w, quad);
+        } else {
+            const float2 x = *reinterpret_cast<const float2 *>(r + 4 * Tab::kPairs);
+            lin = fmaf(u[k][T - 1], x.x, lin);
+            quad = fmaf(u[k][T - 1] * u[k][T - 1], x.y, quad);
+        }
+        quad = fmaf(v * v, cq[k * T * T], quad);
+    }
+    B = quad + (quad2.x + quad2.y);
+    return B + (lin + (lin2.x + lin2.y));
+}
+
+// u of a proposal, one per lane: lane k T + t holds u_t of shell k (S T <= 18
+// lanes; the others 0).  Convergent warp, p and q the same in every lane.
+template <int T, class L, int W>
+__device__ __forceinline__ int pair_diff(const HistEntry<W> &p, const HistEntry<W> &q)
+{
+    constexpr int S = L::S;
+    using H = SiteHist<T, S, L::kImplicit>;
+    const int lane = threadIdx.x & 31, k = lane / T, t = lane - k * T;
+    const bool in = lane < S * T;
+    int u = 0;
+    if (in && t < T - 1) u = hist_field<H>(q, k, t) - hist_field<H>(p, k, t);
+    int rest = 0;
+#pragma unroll
+    for (int i = 0; i < T - 1; ++i) rest += __shfl_sync(0xFFFFFFFFu, u, in ? k * T + i : 0);
+    return in && t == T - 1 ? -rest : u;
+}
+
+// D of the proposal (a, b, p, q; the same in every lane, m folded in) exactly
+// as the contract orders it, from the counts.  Convergent warp: lane k T + t
+// computes the term of species t in shell k, then every lane runs the sum.
+template <int T, class L, int W>
+__device__ __forceinline__ double exact_delta(const SearchConst &c, const int32_t *cnt, int a, int b, HistEntry<W> p,
+                                           HistEntry<W> q)
+{
+    constexpr int S = L::S;
+    const int lane = threadIdx.x & 31;
+    const bool in = lane < S * T;
+    const int k = in ? lane / T : 0, t = in ? lane - k * T : 0;
+    const int u = pair_diff<T, L>(p, q);
+    const double *R = c.R + k * T * T, *E = c.E + k * T * T;
+    const double Ca = (double)cnt[(k * T + a) * T + t], Cb = (double)cnt[(k * T + b) * T + t];
+    const double Ga = __dmul_rn(R[a * T + t], __dadd_rn(__fma_rn(-Ca, R[a * T + t], E[a * T + t]),
+                                                         __fma_rn(-Ca, R[a * T + t], E[t * T + a])));
+    const double Gb = __dmul_rn(R[b * T + t], __dadd_rn(__fma_rn(-Cb, R[b * T + t], E[b * T + t]),
+                                                         __fma_rn(-Cb, R[b * T + t], E[t * T + b])));
+    const double lin = __dmul_rn(__dmul_rn(-2.0, c.w[k]), __dsub_rn(Ga, Gb));
+    const double inner = __fma_rn((double)u, delta_quad<T>(R, c.w[k], a, b, t), lin);
+    double D = 0.0;
+#pragma unroll 1
+    for (int s = 0; s < S; ++s) {
+        for (int i = 0; i < T; ++i)
+            D = __fma_rn((double)__shfl_sync(0xFFFFFFFFu, u, s * T + i), __shfl_sync(0xFFFFFFFFu, inner, s * T + i), D);
+        const int v = __shfl_sync(0xFFFFFFFFu, u, s * T + a) - __shfl_sync(0xFFFFFFFFu, u, s * T + b);
+        D = __fma_rn((double)(v * v), delta_cross<T>(c.R + s * T * T, c.w[s], a, b), D);
+    }
+    return D;
+}
+
+// The same by one lane alone, each of the calling lanes with its own proposal.
+template <int T, class L, int W>
+__device__ __noinline__ double exact_delta_lane(const SearchConst &c, const int32_t *cnt, int ab, HistEntry<W> p,
+                                                HistEntry<W> q)
+{
+    constexpr int S = L::S;
+    using H = SiteHist<T, S, L::kImplicit>;
+    const int a = ab & 0xFF, b = ab >> 8;
     double D = 0.0;
 #pragma unroll
     for (int k = 0; k < S; ++k) {
-        const double2 *e = row + k * T * T * R;
+        const double *R = c.R + k * T * T, *E = c.E + k * T * T, w = c.w[k];
+        int rest = 0, v = 0;
 #pragma unroll
         for (int t = 0; t < T; ++t) {
-            const double u = (double)(field5(h2[k], 5 * t) - field5(h1[k], 5 * t));
-            const double2 lq = e[t];
-            D = __fma_rn(u, __fma_rn(u, lq.y, lq.x), D);
+            const int u = t < T - 1 ? hist_field<H>(q, k, t) - hist_field<H>(p, k, t) : -rest;
+            rest += u;
+            v += ((t == a) - (t == b)) * u;
+            const double Ra = R[a * T + t], Rb = R[b * T + t];
+            const double Ca = (double)cnt[(k * T + a) * T + t], Cb = (double)cnt[(k * T + b) * T + t];
+            const double Ga = __dmul_rn(Ra, __dadd_rn(__fma_rn(-Ca, Ra, E[a * T + t]), __fma_rn(-Ca, Ra, E[t * T + a])));
+            const double Gb = __dmul_rn(Rb, __dadd_rn(__fma_rn(-Cb, Rb, E[b * T + t]), __fma_rn(-Cb, Rb, E[t * T + b])));
+            const double lin = __dmul_rn(__dmul_rn(-2.0, w), __dsub_rn(Ga, Gb));
+            D = __fma_rn((double)u, __fma_rn((double)u, delta_quad<T>(R, w, a, b, t), lin), D);
         }
-        const int v = field5(h2[k], a5) - field5(h1[k], a5) - field5(h2[k], b5) + field5(h1[k], b5);
-        D = __fma_rn((double)(v * v), e[T].x, D);
+        D = __fma_rn((double)(v * v), delta_cross<T>(R, w, a, b), D);
     }
     return D;
+}
+
+// The winner among the warp's candidates whose screened intervals do not
+// settle it: the lanes with `in` hold proposals (task, ab = a | b << 8, p, q; m
+// folded in), and each computes its exact D.  Returns the lane of the lowest D,
+// lowest task on equal D, or -1 when no D < 0.  Convergent warp.
+template <int T, class L, int W>
+__device__ __forceinline__ int resolve(const SearchConst &c, const int32_t *cnt, bool in, int task, int ab,
+                                       const HistEntry<W> &p, const HistEntry<W> &q)
+{
+    uint64_t key = ~0ull;  // ~bits(D) of D < 0: more negative, smaller
+    if (in) {
+        const double D = exact_delta_lane<T, L, W>(c, cnt, ab, p, q);
+        if (D < 0.0) key = ~(uint64_t)__double_as_longlong(D);
+    }
+    __syncwarp();
+    const uint32_t khi = (uint32_t)(key >> 32), klo = (uint32_t)key;
+    const uint32_t hi = __reduce_min_sync(0xFFFFFFFFu, khi);
+    const uint32_t lo = __reduce_min_sync(0xFFFFFFFFu, khi == hi ? klo : 0xFFFFFFFFu);
+    const bool tied = key != ~0ull && khi == hi && klo == lo;
+    const uint32_t first = __reduce_min_sync(0xFFFFFFFFu, tied ? (uint32_t)task : 0xFFFFFFFFu);
+    return __ffs(__ballot_sync(0xFFFFFFFFu, tied && (uint32_t)task == first)) - 1;
+}
+
+// The least float of the warp, as the least of the integers ordered like them.
+__device__ __forceinline__ float warp_min(float x)
+{
+    const int b = __float_as_int(x), m = __reduce_min_sync(0xFFFFFFFFu, b ^ ((b >> 31) & 0x7FFFFFFF));
+    return __int_as_float(m ^ ((m >> 31) & 0x7FFFFFFF));
+}
+
+
+// The best of the records lane i < n holds the i-th of (lo, hi: its screened
+// interval; load(i): the record): its index, or -1 when none improves.
+// Convergent warp.
+template <int T, class L, class Load>
+__device__ __forceinline__ int best_record(const SearchConst &c, const int32_t *cnt, float lo, float hi, int n,
+                                           Load load)
+{
+    const float least = warp_min(hi);
+    const uint32_t cand = __ballot_sync(0xFFFFFFFFu, lo <= least && lo < 0.0f);
+    if ((cand & (cand - 1)) == 0 && (cand == 0 || least < 0.0f)) return __ffs(cand) - 1;
+    const int lane = threadIdx.x & 31;
+    const auto r = load(lane < n ? lane : 0);
+    return resolve<T, L>(c, cnt, (cand >> lane) & 1u, r.task, r.ab, r.p, r.q);
 }
 
 // After an accepted swap of s1 (species a -> b) and s2 (b -> a): update the
 // histograms of every neighbour listed in both rows (block-wide, atomics in
 // L2; the caller's barrier publishes them).  An entry n in shell k of s1's row
 // means s1 is in n's shell k as often, since tables are symmetric per shell.
-// kSpeciesWord: also the species words of s1 and s2, which draw_pair_hist
-// reads; searches whose draws read the occupancy leave them at their recount
-// values.
+// Adds of packed fields are exact in any order: the sum is modulo 2^64 and
+// every final field is in range.
+// kSpecies: also the species bits of s1 and s2, which draw_pair_hist reads;
+// searches whose draws read the occupancy leave them at their recount values.
 // `me` is this thread's index in the block's order of the work (a rotation of
 // threadIdx.x, so that other updates can run on the first warps meanwhile).
-template <class L, bool kSpeciesWord>
-__device__ __forceinline__ void update_hist(const SearchConst &c, const int4 *__restrict__ nbor, uint4 *hist,
+template <int T, class L, bool kSpecies>
+__device__ __forceinline__ void update_hist(const SearchConst &c, const int4 *__restrict__ nbor, uint64_t *hist,
                                             uint32_t s1, uint32_t s2, int a, int b, int me)
 {
-    const uint32_t up = (1u << (5 * b)) - (1u << (5 * a));  // s1's neighbours: one a becomes b
+    using H = SiteHist<T, L::S, L::kImplicit>;
+    unsigned long long *h = reinterpret_cast<unsigned long long *>(hist);
+    // one a becomes b among s1's neighbours, one b becomes a among s2's
+    const auto add = [h, a, b](int n, int k, bool first) {
+        const unsigned long long up = hist_unit<H, T>(k, b) - hist_unit<H, T>(k, a);
+        atomicAdd(h + (size_t)n * H::W + H::word(k, 0), first ? up : 0ull - up);
+    };
     if constexpr (L::kImplicit) {  // row e of s1 then of s2, shells concatenated
         const int row = c.lat.zoff[L::S - 1] + c.lat.zsize[L::S - 1];
         for (int e = me; e < 2 * row; e += blockDim.x) {
@@ -567,36 +990,34 @@ __device__ __forceinline__ void update_hist(const SearchConst &c, const int4 *__
             int k = 0;
 #pragma unroll
             for (int kk = 1; kk < L::S; ++kk) k += idx >= c.lat.zoff[kk];
-            atomicAdd(reinterpret_cast<uint32_t *>(hist + n) + k, first ? up : 0u - up);
+            add(n, k, first);
         }
     } else {
-    const int row4 = L::kRuntime ? c.row4 : L::kRow4;
-    const int row = 4 * row4;
-    for (int e = me; e < 2 * row; e += blockDim.x) {
-        const bool first = e < row;
-        const int idx = first ? e : e - row;
-        const int32_t *r = reinterpret_cast<const int32_t *>(nbor + (size_t)(first ? s1 : s2) * row4);
-        const int n = __ldg(r + idx);
-        if (n >= c.num_sites) continue;  // sentinel padding
-        int k = 0;
+        const int row4 = L::kRuntime ? c.row4 : L::kRow4;
+        const int row = 4 * row4;
+        for (int e = me; e < 2 * row; e += blockDim.x) {
+            const bool first = e < row;
+            const int idx = first ? e : e - row;
+            const int32_t *r = reinterpret_cast<const int32_t *>(nbor + (size_t)(first ? s1 : s2) * row4);
+            const int n = __ldg(r + idx);
+            if (n >= c.num_sites) continue;  // sentinel padding
+            int k = 0;
 #pragma unroll
-        for (int kk = 1; kk < L::S; ++kk) k += idx >= 4 * (L::kRuntime ? c.off4[kk] : L::off(kk));
-        uint32_t *h = reinterpret_cast<uint32_t *>(hist + n) + k;
-        atomicAdd(h, first ? up : 0u - up);
+            for (int kk = 1; kk < L::S; ++kk) k += idx >= 4 * (L::kRuntime ? c.off4[kk] : L::off(kk));
+            add(n, k, first);
+        }
     }
-    }
-    if (kSpeciesWord && me == 0) {
-        hist[s1].w = (uint32_t)(5 * b);
-        hist[s2].w = (uint32_t)(5 * a);
+    if (kSpecies && me == 0) {  // adds, since s1 and s2 may be each other's neighbours
+        const unsigned long long up = hist_species_bits<H>(b) - hist_species_bits<H>(a);
+        atomicAdd(h + (size_t)s1 * H::W + H::W - 1, up);
+        atomicAdd(h + (size_t)s2 * H::W + H::W - 1, 0ull - up);
     }
 }
 
-// The three updates of an accepted swap on different warps where the block has
-// enough of them: the table's L half on warps [0, delta_linear's warps), the
-// new counts on the next warps, the neighbours' histograms after those.  The
-// rotated thread indices (block_rotation) keep every loop covering its work once.
-template <int T, int S>
-__host__ __device__ constexpr int accept_linear_warps() { return (S * T + 32 / T - 1) / (32 / T); }
+// The updates of an accepted swap run on different warps where the block has
+// enough of them: counts and table on warps [0, DeltaTab::kWarps), the
+// neighbours' histograms on the next.  The rotated thread index keeps the loop
+// covering its work once.
 __device__ __forceinline__ int block_rotation(int by)
 {
     int me = (int)threadIdx.x - by;
@@ -604,131 +1025,144 @@ __device__ __forceinline__ int block_rotation(int by)
     return me;
 }
 
-// Two attempts per Philox call: (x0, x1) then (x2, x3); valid when both draws
-// accept and the species differ (pyhea/cpp/accelerate.cpp:649-655).  With
-// 16-bit draws (draw16), four attempts per call: attempt j takes the low and
-// the high half of word x_j.  differ(u, v) reads the two sites' species.
-template <class Differ>
-__device__ __forceinline__ bool draw_pair_by(const SearchConst &c, uint32_t stream, uint32_t round, uint32_t task,
-                                             Differ &&differ, uint32_t &s1, uint32_t &s2)
+// Attempt j of a Philox call's words: the two sites it draws, and whether both
+// draws accept.  Two 32-bit attempts per call, (x0, x1) then (x2, x3); with 16-bit
+// draws four, attempt j taking the low and the high half of word x_j (a half in
+// the upper 16 bits draws like a 32-bit word: value and remainder of one product).
+template <bool k16>
+__device__ __forceinline__ bool attempt_sites(const SearchConst &c, const uint32_t (&x)[4], int j, uint32_t &u,
+                                              uint32_t &v)
 {
     const uint32_t n = (uint32_t)c.num_sites;
-    if (c.draw16) {
-        for (uint32_t call = 0; call < kPhiloxCallsPerDraw; ++call) {
-            const u32x4 x = philox4x32_10(u32x4{call, task, round, stream}, c.key0, c.key1);
-            const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+    const uint32_t p = k16 ? x[j] << 16 : x[(2 * j) & 3], q = k16 ? x[j] & 0xFFFF0000u : x[(2 * j + 1) & 3];
+    u = __umulhi(p, n);
+    v = __umulhi(q, n);
+    return p * n >= c.reject && q * n >= c.reject;
+}
+
+// The first valid attempt from Philox call `call` on: both draws accept and the
+// species differ (pyhea/cpp/accelerate.cpp:649-655); differ(u, v) reads them.
+template <bool k16, class Differ>
+__device__ __forceinline__ bool draw_pair_from(const SearchConst &c, uint32_t call, uint32_t stream, uint32_t round,
+                                               uint32_t task, Differ &&differ, uint32_t &s1, uint32_t &s2)
+{
+    for (; call < kPhiloxCallsPerDraw; ++call) {
+        const u32x4 y = philox4x32_10(u32x4{call, task, round, stream}, c.key0, c.key1);
+        const uint32_t x[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                uint32_t u, v;
-                if (bounded_draw16(w[j] & 0xFFFFu, n, c.reject16, u) && bounded_draw16(w[j] >> 16, n, c.reject16, v) &&
-                    differ(u, v)) {
-                    s1 = u;
-                    s2 = v;
-                    return true;
-                }
+        for (int j = 0; j < (k16 ? 4 : 2); ++j) {
+            uint32_t u, v;
+            if (attempt_sites<k16>(c, x, j, u, v) && differ(u, v)) {
+                s1 = u;
+                s2 = v;
+                return true;
             }
-        }
-        return false;
-    }
-    for (uint32_t call = 0; call < kPhiloxCallsPerDraw; ++call) {
-        const u32x4 x = philox4x32_10(u32x4{call, task, round, stream}, c.key0, c.key1);
-        uint32_t u, v;
-        if (bounded_draw(x.x, n, c.reject_below, u) && bounded_draw(x.y, n, c.reject_below, v) && differ(u, v)) {
-            s1 = u;
-            s2 = v;
-            return true;
-        }
-        if (bounded_draw(x.z, n, c.reject_below, u) && bounded_draw(x.w, n, c.reject_below, v) && differ(u, v)) {
-            s1 = u;
-            s2 = v;
-            return true;
         }
     }
     return false;
 }
+template <class Differ>
+__device__ __forceinline__ bool draw_pair_by(const SearchConst &c, uint32_t stream, uint32_t round, uint32_t task,
+                                             Differ &&differ, uint32_t &s1, uint32_t &s2)
+{
+    return c.draw16 ? draw_pair_from<true>(c, 0, stream, round, task, differ, s1, s2)
+                    : draw_pair_from<false>(c, 0, stream, round, task, differ, s1, s2);
+}
 
-// Species from the occupancy (5*species bytes).
+// All attempts of the first call at once -- the species of every attempt's sites
+// in one round trip to shared memory, no branch -- then the calls after it.  A
+// warp needs 3 of 4 attempts on average before its last lane has a pair, so the
+// loop's dependent loads cost more than the loads left unused.
+template <bool k16>
+__device__ __forceinline__ bool draw_pair_at_once(const SearchConst &c, uint32_t stream, uint32_t round, uint32_t task,
+                                                  const uint8_t *occ, uint32_t &s1, uint32_t &s2)
+{
+    constexpr int A = k16 ? 4 : 2;
+    const u32x4 y = philox4x32_10(u32x4{0u, task, round, stream}, c.key0, c.key1);
+    const uint32_t x[4] = {y.x, y.y, y.z, y.w};
+    uint32_t u[A], v[A];
+    bool in[A], ok = false;
+#pragma unroll
+    for (int j = 0; j < A; ++j) in[j] = attempt_sites<k16>(c, x, j, u[j], v[j]);
+#pragma unroll
+    for (int j = 0; j < A; ++j) in[j] = (occ[u[j]] != occ[v[j]]) && in[j];
+#pragma unroll
+    for (int j = A - 1; j >= 0; --j)
+        if (in[j]) {
+            s1 = u[j];
+            s2 = v[j];
+            ok = true;
+        }
+    if (!ok)
+        ok = draw_pair_from<k16>(c, 1, stream, round, task,
+                                 [occ](uint32_t i, uint32_t j) { return occ[i] != occ[j]; }, s1, s2);
+    return ok;
+}
+
+// Species from the occupancy: all first attempts at once where it lies in shared memory.
+template <bool kShared>
 __device__ __forceinline__ bool draw_pair(const SearchConst &c, uint32_t stream, uint32_t round, uint32_t task,
-                                          const uint8_t *occ5, uint32_t &s1, uint32_t &s2)
+                                          const uint8_t *occ, uint32_t &s1, uint32_t &s2)
 {
-    return draw_pair_by(c, stream, round, task, [occ5](uint32_t u, uint32_t v) { return occ5[u] != occ5[v]; }, s1, s2);
+    if constexpr (kShared)
+        return c.draw16 ? draw_pair_at_once<true>(c, stream, round, task, occ, s1, s2)
+                        : draw_pair_at_once<false>(c, stream, round, task, occ, s1, s2);
+    return draw_pair_by(c, stream, round, task, [occ](uint32_t u, uint32_t v) { return occ[u] != occ[v]; }, s1, s2);
 }
 
-// One site's histogram entry.  Structures whose histograms are far larger
-// than L2 (hist_stream, set by the host) read them with evict-first loads:
-// random 16-byte DRAM loads run 1.35x faster that way on B200 and the lines
-// they bring do not push out those of structures that do stay in L2; an
-// L2-resident structure keeps the default policy (evict-first lost 3 % there).
-__device__ __forceinline__ uint4 load_hist(const SearchConst &c, const uint4 *h)
-{
-    return c.hist_stream ? __ldcs(h) : __ldcg(h);
-}
-
-// Species from the site histograms' species words (hist[s].w = 5*species):
-// for an occupancy in HBM this makes the two 16-byte L2 loads of an attempt
-// the only memory round trip of a proposal; p, q are the accepted pair's
-// histograms.
+// Species from the site histograms' top bits: for an occupancy in HBM this
+// makes the two loads of an attempt the only memory round trip of a proposal;
+// p, q are the accepted pair's histograms.
+template <class H>
 __device__ __forceinline__ bool draw_pair_hist(const SearchConst &c, uint32_t stream, uint32_t round, uint32_t task,
-                                               const uint4 *hist, uint32_t &s1, uint32_t &s2, uint4 &p, uint4 &q)
+                                               const uint64_t *hist, uint32_t &s1, uint32_t &s2, HistEntry<H::W> &p,
+                                               HistEntry<H::W> &q)
 {
     return draw_pair_by(
         c, stream, round, task,
         [&c, hist, &p, &q](uint32_t u, uint32_t v) {
-            p = load_hist(c, hist + u);
-            q = load_hist(c, hist + v);
-            return p.w != q.w;
+            load_hist_pair<H::W>(c, hist, u, v, p, q);
+            return hist_species<H>(p) != hist_species<H>(q);
         },
         s1, s2);
 }
 
-// Ordering key of a proposal's delta D: ~bits(D) for D < 0 (more negative,
-// smaller key), all ones for a proposal that does not improve (D >= 0) or for
-// no proposal.  The round's winner is the lexicographic (key, task) minimum.
-constexpr uint64_t kNoSwap = ~0ull;
-__device__ __forceinline__ uint64_t delta_key(double D)
+// A site's histogram entry from its shells' species counts (fields of FB bits,
+// one per species, the padding's sentinel entries counted as species 0) and
+// its own species a.
+template <class H, int T, int S, int FB, class X>
+__device__ __forceinline__ HistEntry<H::W> pack_hist(const SearchConst &c, const X (&h)[S], int a)
 {
-    return D < 0.0 ? ~(uint64_t)__double_as_longlong(D) : kNoSwap;
-}
-__device__ __forceinline__ double key_delta(uint64_t key) { return __longlong_as_double((long long)~key); }
-__device__ __forceinline__ bool better(uint64_t k, int q, uint64_t bk, int bq) { return k < bk || (k == bk && q < bq); }
-
-// The warp's lexicographic (key, q) minimum in every lane, q >= 0: three
-// 32-bit warp reductions (high word, low word among the lanes holding the
-// minimal high word, task among the lanes holding the minimal key).
-__device__ __forceinline__ void warp_argmin(uint64_t &key, int &q)
-{
-    const uint32_t hi = (uint32_t)(key >> 32), lo = (uint32_t)key;
-    const uint32_t mhi = __reduce_min_sync(0xFFFFFFFFu, hi);
-    const uint32_t mlo = __reduce_min_sync(0xFFFFFFFFu, hi == mhi ? lo : 0xFFFFFFFFu);
-    const uint32_t mq = __reduce_min_sync(0xFFFFFFFFu, (hi == mhi && lo == mlo) ? (uint32_t)q : 0xFFFFFFFFu);
-    key = ((uint64_t)mhi << 32) | mlo;
-    q = (int)mq;
-}
-
-// Exact site histogram (5-bit field per species) from the recount's 10-bit
-// fields, less the sentinel entries the padding added to species 0.
-template <int T>
-__device__ __forceinline__ uint32_t pack_hist5(uint64_t h10, int pad)
-{
-    uint32_t r = 0;
+    HistEntry<H::W> e{};
+    uint32_t f[H::kHalves] = {};
 #pragma unroll
-    for (int t = 0; t < T; ++t) r |= (uint32_t)((h10 >> (10 * t)) & 1023u) << (5 * t);
-    return r - (uint32_t)pad;
+    for (int k = 0; k < S; ++k)
+#pragma unroll
+        for (int t = 0; t < T - 1; ++t) {
+            uint32_t n = (uint32_t)(h[k] >> (FB * t)) & ((1u << FB) - 1u);
+            if (t == 0) n -= (uint32_t)c.pad[k];
+            f[H::half(k, t)] |= n << H::bit(k, t);
+        }
+#pragma unroll
+    for (int x = 0; x < H::W; ++x) e.w[x] = ((uint64_t)f[2 * x + 1] << 32) | f[2 * x];
+    e.w[H::W - 1] |= hist_species_bits<H>(a);
+    return e;
 }
 
 // ---------------------------------------------------------------------------
 // Block recount of the pair counts of the occupancy in shared memory.
-// With `hist`, also writes every site's histograms: hist[s] = {H_0, H_1, H_2,
-// 5 species(s)}, H_k = sum over s's shell-k neighbours n of 1 << (5
-// species(n)) -- the species histogram of the neighbourhood, one 5-bit field
-// per species -- and the last word the site's own species (5*species).
+// With `hist`, also writes every site's histogram entry (SiteHist).
 // Per-thread packed 10-bit accumulators [T][S], flushed to shared-memory bins
 // every 32 sites (32 sites * 28 entries < 1024).  Sentinel entries land in
 // field 0 and are removed at the end (pad_k * n_i per row i).
+// kNeighbors: which neighbour form the caller's structures have, so that a
+// kernel compiles the walks it can take.
 // ---------------------------------------------------------------------------
-template <int T, int S>
-__device__ void block_recount(const SearchConst &c, const int4 *__restrict__ nbor, const uint8_t *occ5, int32_t *cnt,
-                              uint4 *hist = nullptr)
+enum RecountForm { kRecountTable, kRecountLattice, kRecountEither };
+
+template <int T, int S, RecountForm kNeighbors>
+__device__ void block_recount(const SearchConst &c, const int4 *__restrict__ nbor, const uint8_t *occ, int32_t *cnt,
+                              uint64_t *hist = nullptr)
 {
     for (int x = threadIdx.x; x < S * T * T; x += blockDim.x) cnt[x] = 0;
     __syncthreads();
@@ -752,26 +1186,31 @@ __device__ void block_recount(const SearchConst &c, const int4 *__restrict__ nbo
     };
     int since = 0;
     // one site with its shell histograms h (10-bit fields)
-    const auto site = [&](int s, const uint64_t (&h)[S]) {
-        const int a5 = occ5[s];
-        uint32_t hs[3] = {0u, 0u, 0u};
+    const auto site = [&](int s, const uint64_t (&h)[S], auto form) {
+        using H = SiteHist<T, S, decltype(form)::value>;
+        const int a = occ[s];
 #pragma unroll
-        for (int k = 0; k < S; ++k) {
+        for (int k = 0; k < S; ++k)
 #pragma unroll
             for (int i = 0; i < T; ++i)
-                if (a5 == 5 * i) acc[i][k] += h[k];
-            if (hist) hs[k] = pack_hist5<T>(h[k], c.pad[k]);
+                if (a == i) acc[i][k] += h[k];
+        if (hist) {
+            const HistEntry<H::W> e = pack_hist<H, T, S, 10>(c, h, a);
+#pragma unroll
+            for (int x = 0; x < H::W; ++x) hist[(size_t)s * H::W + x] = e.w[x];
         }
-        if (hist) hist[s] = make_uint4(hs[0], hs[1], hs[2], (uint32_t)a5);
         if (++since == 32) {
             flush();
             since = 0;
         }
     };
-    if (c.lat.L) {  // implicit neighbours (no sentinel padding: pad[k] == 0)
-        lattice_sites<S, uint64_t>(c.lat, threadIdx.x, blockDim.x,
-                                   [occ5](int n) { return 1ull << (2 * occ5[n]); }, site);
-    } else {
+    if (kNeighbors == kRecountLattice || (kNeighbors == kRecountEither && c.lat.L)) {
+        // implicit neighbours (no sentinel padding: pad[k] == 0)
+        if constexpr (kNeighbors != kRecountTable)
+            lattice_sites<S, uint64_t>(c.lat, threadIdx.x, blockDim.x,
+                                       [occ](int n) { return 1ull << (10 * occ[n]); },
+                                       [&site](int s, const uint64_t (&h)[S]) { site(s, h, std::true_type{}); });
+    } else if constexpr (kNeighbors != kRecountLattice) {
         for (int s = threadIdx.x; s < c.num_sites; s += blockDim.x) {
             uint64_t h[S];
 #pragma unroll
@@ -780,11 +1219,11 @@ __device__ void block_recount(const SearchConst &c, const int4 *__restrict__ nbo
                 const int4 *seg = nbor + (size_t)s * c.row4 + c.off4[k];
                 for (int ch = 0; ch < c.chunks[k]; ++ch) {
                     const int4 x = __ldg(seg + ch);
-                    h[k] += (1ull << (2 * occ5[x.x])) + (1ull << (2 * occ5[x.y])) + (1ull << (2 * occ5[x.z])) +
-                            (1ull << (2 * occ5[x.w]));
+                    h[k] += (1ull << (10 * occ[x.x])) + (1ull << (10 * occ[x.y])) + (1ull << (10 * occ[x.z])) +
+                            (1ull << (10 * occ[x.w]));
                 }
             }
-            site(s, h);
+            site(s, h, std::false_type{});
         }
     }
     flush();
@@ -799,12 +1238,12 @@ __device__ void block_recount(const SearchConst &c, const int4 *__restrict__ nbo
 // ---------------------------------------------------------------------------
 // Random occupancy of population position `pos` of generation `generation`:
 // the sorted species layout read through a keyed Feistel permutation (cycle
-// walking).  Writes 5*species into occ5 and, when gocc != nullptr, species
-// into the slot's row in HBM.  Block-cooperative; no barrier inside.
+// walking).  Writes the species into occ and, when gocc != nullptr, also into
+// the slot's row in HBM.  Block-cooperative; no barrier inside.
 // ---------------------------------------------------------------------------
 template <int T>
 __device__ __forceinline__ void generate_occupancy(const SearchConst &c, uint32_t pos, uint32_t generation,
-                                                   uint8_t *occ5, uint8_t *gocc)
+                                                   uint8_t *occ, uint8_t *gocc)
 {
     uint32_t rk[kFeistelRounds];
     const u32x4 w0 = philox4x32_10(u32x4{pos, generation, 0u, kInitStream}, c.key0, c.key1);
@@ -817,7 +1256,7 @@ __device__ __forceinline__ void generate_occupancy(const SearchConst &c, uint32_
         int t = 0;
 #pragma unroll
         for (int i = 1; i < T; ++i) t += (int)(y >= (uint32_t)c.prefix[i]);
-        occ5[s] = (uint8_t)(5 * t);
+        occ[s] = (uint8_t)t;
         if (gocc) gocc[s] = (uint8_t)t;
     }
 }
@@ -829,19 +1268,20 @@ template <int T, int S>
 __global__ void __launch_bounds__(512, 1) generate_kernel(const SearchConst c, const GenArgs g)
 {
     extern __shared__ __align__(16) uint8_t smem[];
-    uint8_t *occ5 = smem;
+    uint8_t *occ = smem;
     int32_t *cnt = reinterpret_cast<int32_t *>(smem + c.occ_stride + 16);
     const int slot = g.order[blockIdx.x];
     uint8_t *gocc = g.occ + (size_t)slot * c.occ_stride;
     const int n = c.num_sites;
     if (g.generate) {
-        generate_occupancy<T>(c, blockIdx.x, g.generation, occ5, gocc);
+        generate_occupancy<T>(c, blockIdx.x, g.generation, occ, gocc);
     } else {
-        for (int s = threadIdx.x; s < n; s += blockDim.x) occ5[s] = (uint8_t)(5 * gocc[s]);
+        for (int s = threadIdx.x; s < n; s += blockDim.x) occ[s] = gocc[s];
     }
-    if (threadIdx.x == 0) occ5[n] = 0;
+    if (threadIdx.x == 0) occ[n] = 0;
     __syncthreads();
-    block_recount<T, S>(c, g.nbor, occ5, cnt, g.hist ? g.hist + (size_t)slot * n : nullptr);
+    block_recount<T, S, kRecountEither>(c, g.nbor, occ, cnt,
+                                        g.hist ? g.hist + (size_t)slot * n * hist_words(T, S, c.lat.L > 0) : nullptr);
     int32_t *gc = g.cnt + (size_t)slot * S * T * T;
     for (int x = threadIdx.x; x < S * T * T; x += blockDim.x) gc[x] = cnt[x];
     if (threadIdx.x == 0) g.f2[slot] = fitness_of_counts<T, S>(c, cnt);
@@ -850,31 +1290,34 @@ __global__ void __launch_bounds__(512, 1) generate_kernel(const SearchConst c, c
 // ---------------------------------------------------------------------------
 // The local parallel search (pyhea/cpp/accelerate.cpp:601-694): one CTA per
 // solution, one lane per task (lanes loop when tasks > blockDim).  Each round
-// every task scores one proposal against the same state (its delta D, see
-// score_delta); the block takes the (D, task) minimum and accepts it iff
-// D < 0; the search ends after `depth` rounds in a row without an accept.
+// every task scores one proposal against the same state (its delta D,
+// screened: see score_delta); the block takes the (D, task) minimum and accepts
+// it iff D < 0; the search ends after `depth` rounds in a row without an accept.
 //
 // One block barrier per round: each warp publishes its best proposal (a
 // SwapRecord, double-buffered by round parity) before the barrier; after it
 // every warp reduces the records itself and writes the winning swap into the
 // occupancy (all threads write the same two bytes).  On an accept the block
 // writes the counts after the swap into the other count buffer, rebuilds the
-// table's L half from them and updates the site histograms; a second barrier
+// table's L from them and updates the site histograms; a second barrier
 // publishes all three before the next round.
 //
 // Shared memory after the occupancy: the delta table, the records, two count
 // buffers (search_smem_tail).
 // ---------------------------------------------------------------------------
-struct SwapRecord {
-    uint64_t key;           // delta_key of the proposal's D
+template <int W>
+struct __align__(16) SwapRecord {
+    float lo, hi;       // the proposal's D is in [lo, hi] (scaled); kNoSwap when there is none
     int32_t task;
     uint32_t s1, s2;
-    int32_t ab;             // species a | b << 8 before the swap
-    uint32_t h1[3], h2[3];  // shell histograms of both sites, m folded in (score_delta)
-    int32_t stop;           // record 0 of a round: the block stops after it (deadline)
+    int32_t ab;         // species a | b << 8 before the swap
+    HistEntry<W> p, q;  // histograms of both sites, m folded in (score_delta)
+    int32_t stop;       // record 0 of a round: the block stops after it (deadline)
     int32_t pad_;
 };
-static_assert(sizeof(SwapRecord) == 56, "SwapRecord layout");
+static_assert(sizeof(SwapRecord<1>) == 48 && sizeof(SwapRecord<2>) == 64, "SwapRecord layout");
+// Bytes of a record for either neighbour form.
+__host__ __device__ constexpr size_t record_bytes(int T, int S) { return hist_words(T, S, false) == 2 ? 64 : 48; }
 
 __host__ __device__ constexpr int mc_ncount_pad(int ncount) { return (ncount + 3) & ~3; }
 
@@ -882,8 +1325,45 @@ __host__ __device__ constexpr int mc_ncount_pad(int ncount) { return (ncount + 3
 // swap records, two count buffers.
 __host__ __device__ constexpr size_t search_smem_tail(int T, int S, int nwarps)
 {
-    return (size_t)16 * delta_entries(T, S) + (size_t)2 * nwarps * sizeof(SwapRecord) +
+    return delta_bytes(T, S) + (size_t)2 * nwarps * record_bytes(T, S) +
            (size_t)2 * 4 * mc_ncount_pad(S * T * T);
+}
+
+// [lo, hi] of a proposal's D from its screened value and B; both kNoSwap when
+// there is no proposal or its D >= 0 for certain.
+template <int T, int S>
+__device__ __forceinline__ void screen_interval(const SearchConst &c, const DeltaTab<T, S> tab, bool ok, float D,
+                                                float B, float &lo, float &hi)
+{
+    const float4 z4 = *reinterpret_cast<const float4 *>(tab.f + DeltaTab<T, S>::kZ);
+    const float z = fmaxf(fmaxf(z4.x, z4.y), fmaxf(z4.z, z4.w));
+    const float e = fmaf(kScreenEps, fmaf(sqrt_approx(B), z, B), c.screen_floor);
+    ok = ok && D < e;
+    lo = ok ? D - e : kNoSwap;
+    hi = ok ? D + e : kNoSwap;
+}
+
+// Folds the warp's proposals of one pass (lane: r) into its best record of the
+// round, `mine` (in shared memory; `more`: it may hold an earlier pass's).
+// Convergent warp.
+template <int T, class L, class Record>
+__device__ __forceinline__ void keep_best(const SearchConst &c, const int32_t *cnt, Record &mine, const Record &r,
+                                          bool more)
+{
+    const float least = warp_min(r.hi);
+    const uint32_t cand = __ballot_sync(0xFFFFFFFFu, r.lo <= least && r.lo < 0.0f);
+    if (cand) {
+        const int lane = threadIdx.x & 31;
+        int win = __ffs(cand) - 1;
+        if (cand & (cand - 1)) win = resolve<T, L>(c, cnt, (cand >> lane) & 1u, r.task, r.ab, r.p, r.q);
+        if (lane == win) {
+            bool take = !more || r.hi < mine.lo;
+            if (!take && r.lo <= mine.hi)  // an earlier pass's best too near to tell; on equal D it has the lower task
+                take = exact_delta_lane<T, L>(c, cnt, r.ab, r.p, r.q) < exact_delta_lane<T, L>(c, cnt, mine.ab, mine.p, mine.q);
+            if (take) mine = r;
+        }
+    }
+    __syncwarp();
 }
 
 struct McTrace {
@@ -893,7 +1373,7 @@ struct McTrace {
 };
 
 struct McTally {
-    double f2;                       // recomputed from the counts, or the running f2 when yielded
+    double f2;  // recomputed from the counts, or the running f2 of a yielded search with a tolerance
     int64_t rounds, accepts, evals;  // rounds run by this call
     int64_t round_end;               // round index the search continues from
     int miss;                        // consecutive rejections at round_end
@@ -911,127 +1391,120 @@ struct McResume {
     double tol2;                     // kYield: the search ends once its running f2 <= tol2 (< 0: never)
 };
 
-// Count change dC_ij of shell k for the accepted swap in record w (a -> b at
-// s1, b -> a at s2): sa_i u_j + sa_j u_i with u from the record's histograms.
+// Count change dC_ij of shell k for a swap of species a and b with the lanes'
+// u of pair_diff: sa_i u_j + sa_j u_i.  Convergent warp.
 template <int T>
-__device__ __forceinline__ int count_change(const SwapRecord &w, int a, int b, int k, int i, int j)
+__device__ __forceinline__ int count_change(int u, int a, int b, int k, int i, int j)
 {
-    const uint32_t h1 = w.h1[k], h2 = w.h2[k];
-    const int ui = field5(h2, 5 * i) - field5(h1, 5 * i), uj = field5(h2, 5 * j) - field5(h1, 5 * j);
+    const int ui = __shfl_sync(0xFFFFFFFFu, u, k * T + i), uj = __shfl_sync(0xFFFFFFFFu, u, k * T + j);
     return ((i == a) - (i == b)) * uj + ((j == a) - (j == b)) * ui;
 }
 
+// The accept's new counts and L of the table, on the block's first warps
+// (DeltaTab::kWarps).
+template <int T, class L, class R>
+__device__ __forceinline__ void accept_counts(const DeltaTab<T, L::S> tab, const R &w, int a, int b,
+                                              const int32_t *cold, int32_t *cnew)
+{
+    using Tab = DeltaTab<T, L::S>;
+    if ((int)(threadIdx.x >> 5) >= Tab::kWarps) return;
+    const int u = pair_diff<T, L>(w.p, w.q);
+    delta_linear<T, L::S>(tab, cnew, [cold, u, a, b](int k, int i, int j) {
+        return cold[(k * T + i) * T + j] + count_change<T>(u, a, b, k, i, j);
+    });
+}
+
 // Delta table of a search starting from the counts in buffer 0 of cnt2
-// (the two halves of each entry are written by different threads, so one
-// barrier at the end covers both).  Block-wide.
+// Block-wide.
 template <int T, int S>
-__device__ __forceinline__ void search_setup(const SearchConst &c, const int32_t *cnt2, double2 *tab)
+__device__ __forceinline__ void search_setup(const SearchConst &c, const int32_t *cnt2, const DeltaTab<T, S> tab)
 {
     delta_consts<T, S>(c, tab);
-    delta_linear<T, S>(c, tab, [cnt2](int k, int i, int j) { return cnt2[(k * T + i) * T + j]; });
+    __syncthreads();  // the lanes' constants
+    delta_linear<T, S>(tab, nullptr, [cnt2](int k, int i, int j) { return cnt2[(k * T + i) * T + j]; });
     __syncthreads();
 }
 
-// Rounds of the local search on the staged state: occupancy occ5, counts in
+// Rounds of the local search on the staged state: occupancy occ, counts in
 // buffer 0 of cnt2, the delta table tab (search_setup), running f2 `cur`.
 // Every thread returns the same tally; evals is this thread's count.  No
-// barrier at entry.  occ5 may be shared or global memory; every thread writes
-// the accepted swap's bytes itself, so its own later loads see them either
-// way.  The draws read the species from occ5; proposals are scored from the
+// barrier at entry.  occ is in shared memory (kShared) or global memory.  The
+// draws read the species from occ; proposals are scored from the
 // site histograms `hist`, which an accept updates.
-template <int T, class L, bool kYield = false>
-__device__ __forceinline__ McTally mc_rounds(const SearchConst &c, const int4 *__restrict__ nbor, uint8_t *occ5,
-                                             int32_t *cnt2, double2 *tab, SwapRecord *rec, uint32_t stream,
+template <int T, class L, bool kShared, bool kYield = false>
+__device__ __forceinline__ McTally mc_rounds(const SearchConst &c, const int4 *__restrict__ nbor, uint8_t *occ,
+                                             int32_t *cnt2, const DeltaTab<T, L::S> tab, void *records, uint32_t stream,
                                              double cur, int tasks, int depth, int64_t max_rounds, McTrace tr,
-                                             McResume rs, uint4 *hist, const uint32_t *nbmask)
+                                             McResume rs, uint64_t *hist, const uint32_t *nbmask)
 {
     constexpr int S = L::S, NC = S * T * T, NCP = mc_ncount_pad(NC);
+    constexpr int W = SiteHist<T, S, L::kImplicit>::W;
+    using Record = SwapRecord<W>;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    Record *rec = static_cast<Record *>(records);  // [2][nwarps]
     int miss = rs.miss0, buf = 0;
-    int64_t round = rs.round0, accepts = 0, evals = 0;
+    int64_t round = rs.round0, accepts = 0;
+    uint32_t undrawn = 0;  // this thread's tasks that found no pair
     bool yielded = false;
+    // the running f2 adds exact D's; nothing else needs them
+    const bool track = tr.records || (kYield && rs.tol2 >= 0.0);
     while (miss < depth && round < max_rounds && !(kYield && cur <= rs.tol2)) {
-        SwapRecord *rr = rec + (round & 1) * nwarps;
-        SwapRecord &mine = rr[warp];  // this warp's best proposal of the round
-        if (lane == 0) {
-            mine.key = kNoSwap;
-            mine.task = 0x7FFFFFFF;
-        }
+        Record *rr = rec + (round & 1) * nwarps;
+        Record &mine = rr[warp];  // this warp's best proposal of the round
+        if (lane == 0) mine.lo = mine.hi = kNoSwap;
         __syncwarp();
+        const int32_t *cold = cnt2 + buf * NCP;
         // passes of blockDim tasks; lane q of a pass scores task q (warp-uniform trip count)
         for (int q0 = warp * 32; q0 < tasks; q0 += blockDim.x) {
             const int q = q0 + lane;
-            uint32_t s1 = 0, s2 = 0;
-            const bool ok = q < tasks && draw_pair(c, stream, (uint32_t)round, (uint32_t)q, occ5, s1, s2);
+            uint32_t s1 = 0, s2 = 0;  // a lane without a pair scores site 0 with itself and drops the result
+            const bool ok = q < tasks && draw_pair<kShared>(c, stream, (uint32_t)round, (uint32_t)q, occ, s1, s2);
             __syncwarp();  // lanes that needed more draws rejoin before scoring
-            uint64_t key = kNoSwap;
-            uint32_t h1[S], h2[S];
-            int a = 0, b = 0;
-            if (ok) {
-                ++evals;
-                a = occ5[s1] / 5;
-                b = occ5[s2] / 5;
-                key = delta_key(score_delta<T, L>(c, nbor, nbmask, tab, load_hist(c, hist + s1), load_hist(c, hist + s2), s1, s2,
-                                                  a, b, h1, h2));
-            }
-            uint64_t wk = key;
-            int wq = key != kNoSwap ? q : 0x7FFFFFFF;
-            warp_argmin(wk, wq);
-            // the lane holding the pass minimum folds it into the warp's record
-            if (key != kNoSwap && wq == q && better(wk, wq, mine.key, mine.task)) {
-                SwapRecord r;
-                r.key = wk;
-                r.task = wq;
-                r.s1 = s1;
-                r.s2 = s2;
-                r.ab = a | (b << 8);
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    r.h1[k] = k < S ? h1[k < S ? k : 0] : 0;
-                    r.h2[k] = k < S ? h2[k < S ? k : 0] : 0;
-                }
-                r.stop = 0;
-                r.pad_ = 0;
-                mine = r;
-            }
-            __syncwarp();
+            undrawn += q < tasks && !ok;
+            Record r;
+            load_hist_pair<W>(c, hist, s1, s2, r.p, r.q);
+            const int a = occ[s1], b = occ[s2];
+            r.ab = a | (b << 8);
+            float B;
+            const float D = score_delta<T, L>(c, nbor, nbmask, tab, r.p, r.q, s1, s2, a, b, B);
+            screen_interval(c, tab, ok, D, B, r.lo, r.hi);
+            r.task = q;
+            r.s1 = s1;
+            r.s2 = s2;
+            r.stop = 0;
+            r.pad_ = 0;
+            keep_best<T, L>(c, cold, mine, r, q0 != warp * 32);
         }
         // the stop decision travels in warp 0's record (read by all after the barrier)
         if (kYield && tid == 0) rr[0].stop = (rs.deadline_ns && global_ns() >= rs.deadline_ns) ? 1 : 0;
         __syncthreads();
         const bool stop = kYield && rr[0].stop != 0;
         // every warp reduces the records of all warps
-        uint64_t xk = lane < nwarps ? rr[lane].key : kNoSwap;
-        int xq = lane < nwarps ? rr[lane].task : 0x7FFFFFFF;
-        const uint64_t own_k = xk;
-        const int own_q = xq;
-        warp_argmin(xk, xq);
-        if (xk != kNoSwap) {
-            // the record holding the minimum (tasks of records are distinct)
-            const int xw = __ffs(__ballot_sync(0xFFFFFFFFu, own_k == xk && own_q == xq)) - 1;
-            const SwapRecord &w = rr[xw];
-            const int a = w.ab & 0xFF, b = (w.ab >> 8) & 0xFF;
-            occ5[w.s1] = (uint8_t)(5 * b);  // same bytes from every thread
-            occ5[w.s2] = (uint8_t)(5 * a);
-            const int32_t *cold = cnt2 + buf * NCP;
+        const int xw = best_record<T, L>(c, cold, lane < nwarps ? rr[lane].lo : kNoSwap,
+                                         lane < nwarps ? rr[lane].hi : kNoSwap, nwarps,
+                                         [rr](int i) -> const Record & { return rr[i]; });
+        if (xw >= 0) {
+            const Record &w = rr[xw];
+            const int a = w.ab & 0xFF, b = w.ab >> 8;
+            if (tid == 0) {  // read again only after the barrier below
+                occ[w.s1] = (uint8_t)b;
+                occ[w.s2] = (uint8_t)a;
+            }
             int32_t *cnew = cnt2 + (buf ^ 1) * NCP;
-            const auto after = [cold, &w, a, b](int k, int i, int j) {
-                return cold[(k * T + i) * T + j] + count_change<T>(w, a, b, k, i, j);
-            };
-            const int me = block_rotation(32 * accept_linear_warps<T, S>());
-            for (int x = me; x < NC; x += blockDim.x) cnew[x] = after(x / (T * T), (x / T) % T, x % T);
-            delta_linear<T, S>(c, tab, after);
-            update_hist<L, false>(c, nbor, hist, w.s1, w.s2, a, b,
-                                  block_rotation(32 * (accept_linear_warps<T, S>() + (NC + 31) / 32)));
-            const double D = key_delta(xk);
+            accept_counts<T, L>(tab, w, a, b, cold, cnew);
+            update_hist<T, L, false>(c, nbor, hist, w.s1, w.s2, a, b, block_rotation(32 * DeltaTab<T, S>::kWarps));
+            if (track && warp == nwarps - 1) {
+                const double D = exact_delta<T, L>(c, cold, a, b, w.p, w.q);
+                if (lane == 0) *tab.accepted() = D;
+            }
             __syncthreads();  // next round's proposals read the new table and histograms
             buf ^= 1;
-            cur = __dadd_rn(cur, D);
+            if (track) cur = __dadd_rn(cur, *tab.accepted());
             if (tr.records && warp == 0 && accepts < tr.cap) {
                 if (lane == 0) {
                     AcceptRecord r;
                     r.round = (uint32_t)round;
-                    r.task = (uint32_t)xq;
+                    r.task = (uint32_t)rr[xw].task;
                     r.s1 = rr[xw].s1;
                     r.s2 = rr[xw].s2;
                     r.f2 = cur;
@@ -1054,47 +1527,21 @@ __device__ __forceinline__ McTally mc_rounds(const SearchConst &c, const int4 *_
         }
     }
     __syncthreads();
-    const double f2 = yielded ? cur : fitness_of_counts<T, S>(c, cnt2 + buf * NCP);
+    const int64_t scored = (int64_t)(tid < tasks ? (tasks - 1 - tid) / (int)blockDim.x + 1 : 0) * (round - rs.round0);
+    const int64_t evals = scored - undrawn;
+    const double f2 = yielded && track ? cur : fitness_of_counts<T, S>(c, cnt2 + buf * NCP);
     return McTally{f2, round - rs.round0, accepts, evals, round, miss, buf, yielded};
 }
 
-// Slot row (species bytes) -> 5*species in shared memory (16-byte vectors).
-// kFromL2: load through L2 only (rows written earlier by other CTAs of the
-// same launch may sit stale in this SM's L1).
+// One occupancy row to another (16-byte vectors).  kFromL2: load through L2 only
+// (rows written earlier by other CTAs of the same launch may sit stale in this
+// SM's L1); a row copied onto itself that way is fresh in L1 afterwards.
 template <bool kFromL2 = false>
-__device__ __forceinline__ void stage_occupancy(const SearchConst &c, const uint8_t *gocc, uint8_t *occ5)
+__device__ __forceinline__ void copy_occupancy(const SearchConst &c, const uint8_t *from, uint8_t *to)
 {
-    const uint4 *src = reinterpret_cast<const uint4 *>(gocc);
-    uint4 *dst = reinterpret_cast<uint4 *>(occ5);
-    for (int v = threadIdx.x; v < c.occ_stride / 16; v += blockDim.x) {
-        uint4 x = kFromL2 ? __ldcg(src + v) : src[v];
-        // bytes are species < 8: 5*t per byte without carries
-        x.x = x.x * 5u; x.y = x.y * 5u; x.z = x.z * 5u; x.w = x.w * 5u;
-        dst[v] = x;
-    }
-}
-
-// 5*species in shared memory -> slot row (species bytes).
-__device__ __forceinline__ void unstage_occupancy(const SearchConst &c, const uint8_t *occ5, uint8_t *gocc)
-{
-    const uint4 *src = reinterpret_cast<const uint4 *>(occ5);
-    uint4 *dst = reinterpret_cast<uint4 *>(gocc);
-    for (int v = threadIdx.x; v < c.occ_stride / 16; v += blockDim.x) {
-        uint4 x = src[v];
-        // every byte holds 5*t with t < 8: t = (5t * 205) >> 10 per byte
-        uint32_t o[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            uint32_t r = 0;
-#pragma unroll
-            for (int by = 0; by < 4; ++by) {
-                const uint32_t b5 = (o[w] >> (8 * by)) & 0xFFu;
-                r |= ((b5 * 205u) >> 10) << (8 * by);
-            }
-            o[w] = r;
-        }
-        dst[v] = make_uint4(o[0], o[1], o[2], o[3]);
-    }
+    const uint4 *src = reinterpret_cast<const uint4 *>(from);
+    uint4 *dst = reinterpret_cast<uint4 *>(to);
+    for (int v = threadIdx.x; v < c.occ_stride / 16; v += blockDim.x) dst[v] = kFromL2 ? __ldcg(src + v) : src[v];
 }
 
 // Sum of per-thread evaluation counts of the block, added to stats[1];
@@ -1116,25 +1563,26 @@ __device__ __forceinline__ void add_tally(const McTally &t, unsigned long long *
 #endif
 // Shared memory: occ_stride + 16 + search_smem_tail(T, S, nwarps).
 template <int T, class L>
-__global__ void __launch_bounds__(512, HEA_MC_MIN_BLOCKS) mc_kernel(const SearchConst c, const McArgs g)
+__global__ void __launch_bounds__(512, HEA_MC_MIN_BLOCKS) mc_kernel(const __grid_constant__ SearchConst c,
+                                                                               const McArgs g)
 {
     constexpr int S = L::S, NC = S * T * T, NCP = mc_ncount_pad(NC);
     extern __shared__ __align__(16) uint8_t smem[];
     const int tid = threadIdx.x, nwarps = blockDim.x >> 5;
-    uint8_t *occ5 = smem;
-    double2 *tab = reinterpret_cast<double2 *>(smem + c.occ_stride + 16);
-    SwapRecord *rec = reinterpret_cast<SwapRecord *>(tab + delta_entries(T, S));  // [2][nwarps]
-    int32_t *cnt2 = reinterpret_cast<int32_t *>(rec + 2 * nwarps);                // [2][NCP]
+    uint8_t *occ = smem;
+    const DeltaTab<T, S> tab{reinterpret_cast<float *>(smem + c.occ_stride + 16)};
+    uint8_t *rec = reinterpret_cast<uint8_t *>(tab.f + DeltaTab<T, S>::kFloats);         // [2][nwarps] records
+    int32_t *cnt2 = reinterpret_cast<int32_t *>(rec + 2 * nwarps * record_bytes(T, S));  // [2][NCP]
 
     const int slot = g.order[blockIdx.x];
     const uint32_t stream = (g.mc_call << 16) | (uint32_t)blockIdx.x;
     uint8_t *gocc = g.occ + (size_t)slot * c.occ_stride;
     int32_t *gcnt = g.cnt + (size_t)slot * NC;
 
-    stage_occupancy(c, gocc, occ5);
+    copy_occupancy(c, gocc, occ);
     for (int x = tid; x < NC; x += blockDim.x) cnt2[x] = gcnt[x];
     __syncthreads();
-    if (tid == 0) occ5[c.num_sites] = 0;  // sentinel (occ_stride may end exactly at n)
+    if (tid == 0) occ[c.num_sites] = 0;  // sentinel (occ_stride may end exactly at n)
     search_setup<T, S>(c, cnt2, tab);
 
     McTrace tr{nullptr, nullptr, 0};
@@ -1143,11 +1591,12 @@ __global__ void __launch_bounds__(512, HEA_MC_MIN_BLOCKS) mc_kernel(const Search
         tr.counts = g.trace_counts ? g.trace_counts + (size_t)blockIdx.x * g.trace_cap * NC : nullptr;
         tr.cap = g.trace_cap;
     }
-    const McTally t = mc_rounds<T, L>(c, g.nbor, occ5, cnt2, tab, rec, stream, g.f2[slot], g.tasks, g.depth,
+    const McTally t = mc_rounds<T, L, true>(c, g.nbor, occ, cnt2, tab, rec, stream, g.f2[slot], g.tasks, g.depth,
                                       g.max_rounds, tr, McResume{0, 0, 0ull, -1.0},
-                                      g.hist + (size_t)slot * c.num_sites, g.nbmask);
+                                      g.hist + (size_t)slot * c.num_sites * hist_words(T, S, L::kImplicit),
+                                      g.nbmask);
 
-    unstage_occupancy(c, occ5, gocc);
+    copy_occupancy(c, occ, gocc);
     for (int x = tid; x < NC; x += blockDim.x) gcnt[x] = cnt2[t.buf * NCP + x];
     add_tally(t, g.stats);
     if (tid == 0) {

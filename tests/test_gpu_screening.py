@@ -1,0 +1,76 @@
+"""Proposals are screened in FP32 and decided exactly: whole searches equal the
+oracle bit for bit where the screening's choices are hardest -- many equal D's
+(two species, one shell), a species of a single atom, targets already met,
+weights or targets outside FP32's range, six species in three shells (both
+histogram widths) -- and where a round takes several passes (CTAs smaller than
+the round, on one CTA and on a cluster, in both draw modes)."""
+import numpy as np
+import pytest
+
+import pyhea_b200 as hb
+from oracle import hea_oracle as ho
+from pyhea_b200 import lattice as L
+from pyhea_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def problems(lattice, cell, species, shells, shell_set=L.SHELLS_REFERENCE, seed=0, weight=None, scale=1.0, recognize=True):
+    st = W.small_case(lattice=lattice, cell=cell, species=species, shells=shells, shell_set=shell_set, seed=seed)
+    nbor, sizes = st.neighbors()
+    weight = st.weight if weight is None else weight
+    target = scale * np.asarray(st.target)
+    row = int(sizes[:shells].sum())
+    return (hb.Problem(nbor, sizes, st.species, weight, target, recognize=recognize),
+            ho.Problem(nbor[:, :row], sizes[:shells], st.species, weight, target))
+
+
+def same(gp, op, P, I, Q, D, seed, **kw):
+    occ, fit, stats = hb.search(gp, P, I, Q, D, seed=seed, **kw)
+    kw.pop("hbm_occupancy", None)
+    wocc, wf2, wstats = op.hcs(seed, P, I, Q, D, **kw)
+    np.testing.assert_array_equal(occ, wocc)
+    np.testing.assert_array_equal(fit, np.sqrt(wf2))
+    assert (stats["evals"], stats["accepts"], stats["rounds"]) == (wstats["evals"], wstats["accepts"], wstats["rounds"])
+
+
+@pytest.mark.parametrize("species,shells,weight,scale", [
+    ((128, 128), 1, None, 1.0),            # few distinct D's: ties in every round
+    ((255, 1), 2, None, 1.0),              # one atom of a species
+    ((100, 100, 55, 1), 3, None, 1.0),
+    ((86, 85, 85), 3, None, 0.0),          # target of random structures: D near 0
+    ((64, 64, 64, 64), 3, [1e-40, 1e-41, 1e-42], 1.0),
+    ((64, 64, 64, 64), 3, [1e30, 1.0, 1e-30], 1.0),
+    ((64, 64, 64, 64), 3, [1e-300, 1.0, 1e300], 1.0),  # beyond FP32's range: every proposal exact
+    ((64, 64, 64, 64), 3, [0.0, 1.0, 0.0], 1.0),
+    ((64, 64, 64, 64), 3, [0.0, 0.0, 0.0], 1.0),
+    ((64, 64, 64, 64), 3, None, 1e9),      # targets far outside
+])
+@pytest.mark.parametrize("hbm", [False, True])
+def test_hard_choices(species, shells, weight, scale, hbm):
+    gp, op = problems(L.FCC, 4, species, shells, seed=len(species), weight=weight, scale=scale)
+    same(gp, op, 3, 2, 96, 3, seed=77, max_rounds=150, hbm_occupancy=hbm)
+
+
+@pytest.mark.parametrize("lattice,shell_set", [(L.FCC, L.SHELLS_FCC_TRUE3), (L.FCC, L.SHELLS_REFERENCE), (L.BCC, 0)])
+@pytest.mark.parametrize("recognize", [True, False])
+@pytest.mark.parametrize("hbm", [False, True])
+def test_six_species(lattice, shell_set, recognize, hbm):
+    n = L.num_sites(lattice, 5)
+    species = W.dirichlet_counts(np.random.default_rng(6), 6, n)
+    gp, op = problems(lattice, 5, species, 3, shell_set, seed=2, recognize=recognize)
+    same(gp, op, 3, 2, 200, 4, seed=9, hbm_occupancy=hbm)
+
+
+@pytest.mark.parametrize("tasks", [257, 400, 512, 600, 769])
+def test_passes_of_small_ctas(tasks):
+    """More solutions in flight than one CTA of 512 threads per SM pair: CTAs of at most 256 threads."""
+    gp, op = problems(L.BCC, 3, (20, 17, 17), 2, seed=tasks)
+    same(gp, op, 75, 8, tasks, 2, seed=tasks)
+
+
+@pytest.mark.parametrize("cell,tasks", [(6, 9000), (27, 8200), (27, 4097)])
+def test_passes_on_a_cluster(cell, tasks):
+    n = L.num_sites(L.FCC, cell)
+    gp, op = problems(L.FCC, cell, [n // 4] * 4, 3, L.SHELLS_FCC_TRUE3, seed=1)
+    same(gp, op, 2, 1, tasks, 3, seed=5, max_rounds=25, hbm_occupancy=True)

@@ -3,12 +3,15 @@
 
 namespace hea {
 
-// Stable ascending order of order[0, count) by f2 (rank counting); block-wide,
-// barriers inside.  scratch holds `count` ints.  Reads go through L2: the
-// values were written by other CTAs of the same launch.
-__device__ __forceinline__ void block_stable_sort(int32_t *order, const double *f2, int count, int32_t *scratch)
+// Stable ascending order by f2 (rank counting) of the slots a[0, na) followed by
+// b[0, nb), both rewritten in rank order; block-wide, barriers inside.  scratch
+// holds na + nb ints.  Reads go through L2: the values were written by other
+// CTAs of the same launch.
+__device__ __forceinline__ void block_stable_sort(int32_t *a, int na, int32_t *b, int nb, const double *f2,
+                                                  int32_t *scratch)
 {
-    for (int i = threadIdx.x; i < count; i += blockDim.x) scratch[i] = __ldcg(order + i);
+    const int count = na + nb;
+    for (int i = threadIdx.x; i < count; i += blockDim.x) scratch[i] = __ldcg(i < na ? a + i : b + (i - na));
     __syncthreads();
     for (int i = threadIdx.x; i < count; i += blockDim.x) {
         const double fi = __ldcg(f2 + __ldcg(scratch + i));
@@ -17,26 +20,28 @@ __device__ __forceinline__ void block_stable_sort(int32_t *order, const double *
             const double fj = __ldcg(f2 + __ldcg(scratch + j));
             r += (fj < fi) || (fj == fi && j < i);
         }
-        order[r] = __ldcg(scratch + i);
+        *(r < na ? a + r : b + (r - na)) = __ldcg(scratch + i);
     }
     __threadfence();
     __syncthreads();
 }
+
+__device__ __forceinline__ int job_ring(int level, int kind) { return 2 * level + (kind == kJobGenMc); }
 
 __device__ __forceinline__ BatchJob &ring_slot(BatchJob *jobs, const BatchQueue &q, unsigned long long h)
 {
     return jobs[q.base + h % q.cap];
 }
 
-// Append `n` fresh jobs of one kind for structure s to ring `level`
+// Append `n` fresh jobs of one kind for structure s to its ring of `level`
 // (block-wide; thread 0 reserves the positions).
 __device__ __forceinline__ void enqueue_jobs(BatchJob *jobs, BatchCtl *ctl, int level, int s, int kind, int iter,
                                              int n, unsigned long long *first_sh)
 {
-    if (threadIdx.x == 0) *first_sh = atomicAdd(&ctl->q[level].tail, (unsigned long long)n);
+    BatchQueue &q = ctl->q[job_ring(level, kind)];
+    if (threadIdx.x == 0) *first_sh = atomicAdd(&q.tail, (unsigned long long)n);
     __syncthreads();
     const unsigned long long first = *first_sh;
-    const BatchQueue &q = ctl->q[level];
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const unsigned long long h = first + i;
         BatchJob &j = ring_slot(jobs, q, h);
@@ -57,8 +62,9 @@ __device__ __forceinline__ void enqueue_jobs(BatchJob *jobs, BatchCtl *ctl, int 
 __device__ __forceinline__ void enqueue_resume(BatchJob *jobs, BatchCtl *ctl, int level, const BatchJob &job,
                                                int64_t round0, int miss0)
 {
-    const unsigned long long h = atomicAdd(&ctl->q[level].tail, 1ull);
-    BatchJob &j = ring_slot(jobs, ctl->q[level], h);
+    BatchQueue &q = ctl->q[job_ring(level, job.kind)];
+    const unsigned long long h = atomicAdd(&q.tail, 1ull);
+    BatchJob &j = ring_slot(jobs, q, h);
     j.structure = job.structure;
     j.kind = job.kind;
     j.index = job.index;
@@ -70,39 +76,60 @@ __device__ __forceinline__ void enqueue_resume(BatchJob *jobs, BatchCtl *ctl, in
     atomicExch(&j.seq, (int32_t)(uint32_t)(h + 1));
 }
 
-// Thread 0: take the next reserved job of the highest level that has one.
-// Returns its slot and expected sequence number, or -1 when no structure is
-// active, the deadline has passed, or on error.
+// The block's first warp, converged: take the next reserved job of the first
+// ring that has one; lane l looks at ring l, so a look costs one round trip to
+// L2 however far down the work is.  Returns its slot and expected sequence
+// number (every lane), or -1 when no structure is active, the deadline has
+// passed, or on error.
 __device__ __forceinline__ long long claim_job(BatchCtl *ctl, unsigned long long deadline, int32_t *seq)
 {
+    const int lane = threadIdx.x & 31;
     const unsigned long long t0 = global_ns();
+    volatile BatchQueue *q = &ctl->q[lane];
     for (;;) {
-        if (*(volatile int32_t *)&ctl->active <= 0 || *(volatile int32_t *)&ctl->error) return -1;
-        const unsigned long long now = global_ns();
-        if (deadline && now >= deadline) return -1;
-        for (int l = 0; l < kBatchLevels; ++l) {
-            volatile BatchQueue *q = &ctl->q[l];
-            unsigned long long h = q->head;
-            while (h < q->tail) {
-                const unsigned long long old = atomicCAS(&ctl->q[l].head, h, h + 1);
-                if (old == h) {
-                    *seq = (int32_t)(uint32_t)(h + 1);
-                    return (long long)(q->base + h % q->cap);
+        // head before tail: the pair never shows a job that was not reserved
+        const unsigned long long head = q->head, tail = q->tail;
+        int out = 0;  // lane 0: why to stop
+        unsigned long long now = 0;
+        if (lane == 0) {
+            now = global_ns();
+            if (*(volatile int32_t *)&ctl->active <= 0 || *(volatile int32_t *)&ctl->error || (deadline && now >= deadline))
+                out = 1;
+        }
+        if (__shfl_sync(0xFFFFFFFFu, out, 0)) return -1;
+        const uint32_t ready = __ballot_sync(0xFFFFFFFFu, head < tail);
+        if (ready) {
+            const int ring = __ffs(ready) - 1;
+            unsigned long long mine = head;
+            int won = 0;
+            if (lane == ring)
+                while (!won && mine < tail) {
+                    const unsigned long long old = atomicCAS(&ctl->q[ring].head, mine, mine + 1);
+                    won = old == mine;
+                    if (!won) mine = old;  // another CTA took it: try the next
                 }
-                h = old;
+            __syncwarp();
+            if (__shfl_sync(0xFFFFFFFFu, won, ring)) {
+                const unsigned long long h = __shfl_sync(0xFFFFFFFFu, mine, ring);
+                *seq = (int32_t)(uint32_t)(h + 1);
+                return (long long)(ctl->q[ring].base + h % ctl->q[ring].cap);
+            }
+            continue;  // others took them all
+        }
+        if (lane == 0) {
+            const unsigned long long prog = *(volatile unsigned long long *)&ctl->progress_ns;
+            const unsigned long long since = prog > t0 ? prog : t0;  // another SM's clock read may be ahead of ours
+            if (now > since && now - since > ctl->wait_limit_ns) {
+                atomicExch(&ctl->error, 1);
+                out = 1;
             }
         }
-        const unsigned long long prog = *(volatile unsigned long long *)&ctl->progress_ns;
-        const unsigned long long since = prog > t0 ? prog : t0;  // another SM's clock read may be ahead of ours
-        if (now > since && now - since > ctl->wait_limit_ns) {
-            atomicExch(&ctl->error, 1);
-            return -1;
-        }
+        if (__shfl_sync(0xFFFFFFFFu, out, 0)) return -1;
         __nanosleep(256);
     }
 }
 
-// Phase-0 jobs of structures list[0, gridDim.x) (all structures when list is
+// First jobs of structures list[0, gridDim.x) (all structures when list is
 // NULL); one CTA per structure.
 __global__ void batch_seed_kernel(const BatchStruct *structs, const int32_t *list, BatchState *states, BatchJob *jobs,
                                   BatchCtl *ctl)
@@ -110,19 +137,25 @@ __global__ void batch_seed_kernel(const BatchStruct *structs, const int32_t *lis
     __shared__ unsigned long long first;
     const int s = list ? list[blockIdx.x] : (int)blockIdx.x;
     const BatchStruct &d = structs[s];
+    const int ahead = min(d.ahead, d.I);
     if (threadIdx.x == 0) {
         BatchState &st = states[s];
-        st.remaining = d.I > 0 ? 2 * d.P : d.P;
+        st.survivors = d.P;
+        for (int r = 0; r < kBatchAhead; ++r) {
+            st.left[r] = r < ahead ? d.P : 0;
+            st.join[r] = 0;
+        }
+        st.iter = -1;
         st.phase = 0;
         st.done = 0;
         st.tally[0] = st.tally[1] = st.tally[2] = 0;
         __threadfence();
         atomicAdd(&ctl->active, 1);
     }
-    for (int i = threadIdx.x; i < 2 * d.P; i += blockDim.x) d.order[i] = i;
+    for (int i = threadIdx.x; i < (d.ahead + 1) * d.P; i += blockDim.x) d.order[i] = i;
     __syncthreads();
     enqueue_jobs(jobs, ctl, d.level, s, kJobGen0, 0, d.P, &first);
-    if (d.I > 0) enqueue_jobs(jobs, ctl, d.level, s, kJobGenMc, 0, d.P, &first);
+    for (int it = 0; it < ahead; ++it) enqueue_jobs(jobs, ctl, d.level, s, kJobGenMc, it, d.P, &first);
 }
 
 struct JobEnd {
@@ -147,7 +180,7 @@ __device__ __noinline__ McTally batch_search(const SearchConst &c, const BatchSt
                                              const DeltaTab<T, L::S> tab, void *rec, uint32_t stream, double cur,
                                              const McResume rs, uint64_t *hist)
 {
-    return mc_rounds<T, L, false, true>(c, d.nbor, occ, cnt2, tab, rec, stream, cur, d.Q, d.D, d.max_rounds,
+    return mc_rounds<T, L, true>(c, d.nbor, occ, cnt2, tab, rec, stream, cur, d.Q, d.D, d.max_rounds,
                                  McTrace{nullptr, nullptr, 0}, rs, hist, d.nbmask);
 }
 
@@ -161,7 +194,7 @@ __device__ __noinline__ JobEnd batch_job(const SearchConst &c, const BatchStruct
     const bool hbm = d.hbm != 0;
     const int P = d.P, n = c.num_sites;
     const int pos = job.index;
-    const int slot = __ldcg(d.order + (job.kind == kJobGenMc ? P + pos : pos));
+    const int slot = __ldcg(d.order + (job.kind == kJobGenMc ? P * (job.iter % d.ahead + 1) + pos : pos));
     uint8_t *gocc = d.occ + (size_t)slot * c.occ_stride;
     int32_t *gcnt = d.cnt + (size_t)slot * NC;
     uint64_t *hist = d.hist + (size_t)slot * c.num_sites * hist_words(T, S, L::kImplicit);
@@ -232,18 +265,16 @@ __global__ void __launch_bounds__(HEA_BATCH_THREADS, HEA_BATCH_MIN_BLOCKS)
 {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ BatchJob job;
-    __shared__ int stop, last, phase;
+    __shared__ int merge, behind;
     __shared__ unsigned long long first;
     __shared__ __align__(16) SearchConst c;  // this job's constants: fitness tables read from shared memory
     const unsigned long long deadline = ctl->deadline_ns;  // set before the launch
     for (;;) {
+        int32_t seq = 0;
+        const long long h = threadIdx.x < 32 ? claim_job(ctl, deadline, &seq) : 0;
+        int stop = h < 0;  // thread 0's counts
         if (threadIdx.x == 0) {
-            stop = 0;
-            int32_t seq = 0;
-            const long long h = claim_job(ctl, deadline, &seq);
-            if (h < 0) {
-                stop = 1;
-            } else {
+            if (h >= 0) {
                 volatile int32_t *vs = &jobs[h].seq;
                 const unsigned long long t0 = global_ns();
                 while (*vs != seq) {  // the producer reserved this position and is filling it
@@ -272,8 +303,10 @@ __global__ void __launch_bounds__(HEA_BATCH_THREADS, HEA_BATCH_MIN_BLOCKS)
                 }
             }
         }
-        __syncthreads();
-        if (stop) break;
+        // A barrier that carries thread 0's answer (not a plain one and a shared flag: between that and
+        // the barrier that ends the loop body only the first warp works, and the other warps were seen to
+        // run the old job again).
+        if (__syncthreads_or(threadIdx.x == 0 && stop)) break;
         // this job's structure: read-only while it is active
         const BatchStruct &d = structs[job.structure];
         {  // 8-byte words: SearchConst holds doubles, so it is 8-byte aligned and sized
@@ -293,37 +326,55 @@ __global__ void __launch_bounds__(HEA_BATCH_THREADS, HEA_BATCH_MIN_BLOCKS)
         }
         __threadfence();  // every writer orders its results before the completion count
         __syncthreads();
+        // the last job of its kind runs the structure's transition; merge: the iteration to merge, or -1
+        const int s = job.structure, P = d.P, I = d.I;
+        BatchState &st = states[s];
+        const bool population = job.kind == kJobGenMc;
+        int last = 0;  // thread 0's counts
         if (threadIdx.x == 0) {
+            merge = -1;
             if (e.yielded) {
                 enqueue_resume(jobs, ctl, d.level, job, e.round, e.miss);
-                last = 0;
             } else {
-                last = atomicSub(&states[job.structure].remaining, 1) == 1;
+                last = atomicSub(population ? &st.left[job.iter % d.ahead] : &st.survivors, 1) == 1;
                 atomicMax(&ctl->progress_ns, global_ns());
-                if (last) {
-                    __threadfence();
-                    phase = __ldcg(&states[job.structure].phase);
+                if (last) __threadfence();
+                if (last && !population) behind = __ldcg(&st.iter) + 1;
+                if (last && population) {
+                    if (atomicAdd(&st.join[job.iter % d.ahead], 1) == 1) merge = job.iter;
                 }
             }
         }
-        __syncthreads();
-        if (!last) continue;
-        // phase transition of this structure
-        const int s = job.structure, P = d.P, I = d.I, k = phase;
-        bool finished = (k == 0 && I == 0);  // generation 0 only: the reference returns it unsorted
+        if (!__syncthreads_or(threadIdx.x == 0 && last)) continue;
+        bool finished = false;
+        if (!population) {
+            // iterations the survivors have behind them, read once: another CTA may merge and count on
+            // as soon as the token below is in
+            const int k = behind;
+            if (k > 0) block_stable_sort(d.order, P, nullptr, 0, d.f2, d.scratch);
+            finished = k == I;  // with I = 0, generation 0 only: the reference returns it unsorted
+            if (!finished && threadIdx.x == 0) {
+                __threadfence();
+                if (atomicAdd(&st.join[k % d.ahead], 1) == 1) merge = k;
+            }
+            if (finished && threadIdx.x == 0) st.phase = k;
+            __syncthreads();
+        }
+        const int it = merge;
+        if (!finished && it < 0) continue;  // the other token comes later
         if (!finished) {
-            if (k > 0) block_stable_sort(d.order, d.f2, P, d.scratch);  // survivors after their search
-            if (k == I)
-                finished = true;
-            else if (k > 0 && d.tol2 >= 0.0 && __ldcg(d.f2 + __ldcg(d.order)) <= d.tol2)
+            __threadfence();
+            if (it > 0 && d.tol2 >= 0.0 && __ldcg(d.f2 + __ldcg(d.order)) <= d.tol2) {
                 finished = true;  // tolerance reached
-            else
-                block_stable_sort(d.order, d.f2, 2 * P, d.scratch);  // merge of iteration k
+                if (threadIdx.x == 0) st.phase = it;
+            } else {
+                block_stable_sort(d.order, P, d.order + (size_t)P * (it % d.ahead + 1), P, d.f2, d.scratch);
+            }
         }
         if (finished) {
             if (threadIdx.x == 0) {
                 finish_ns[s] = global_ns() - ctl->start_ns;
-                states[s].done = 1;
+                st.done = 1;
                 __threadfence();
                 atomicAdd(&ctl->stats[3], 1ull);
                 atomicSub(&ctl->active, 1);
@@ -331,14 +382,17 @@ __global__ void __launch_bounds__(HEA_BATCH_THREADS, HEA_BATCH_MIN_BLOCKS)
             __syncthreads();
             continue;
         }
+        const bool more = it + d.ahead < I;  // another population into the slots the merge freed
         if (threadIdx.x == 0) {
-            states[s].phase = k + 1;
-            states[s].remaining = (k + 1 < I) ? 2 * P : P;
+            st.iter = it;
+            st.survivors = P;
+            st.join[it % d.ahead] = 0;
+            if (more) st.left[it % d.ahead] = P;
             __threadfence();
         }
         __syncthreads();
-        enqueue_jobs(jobs, ctl, d.level, s, kJobMc2, k, P, &first);
-        if (k + 1 < I) enqueue_jobs(jobs, ctl, d.level, s, kJobGenMc, k + 1, P, &first);
+        enqueue_jobs(jobs, ctl, d.level, s, kJobMc2, it, P, &first);
+        if (more) enqueue_jobs(jobs, ctl, d.level, s, kJobGenMc, it + d.ahead, P, &first);
     }
 }
 

@@ -6,27 +6,32 @@
 // Every structure runs the same search as the plain path (hea_search.cuh) with
 // its own constants, tables, population pools and Philox key, so its result
 // is bit-identical to searching it alone, whatever else shares the GPU.  Its
-// work is a sequence of phases of jobs:
+// work is a graph of jobs, P of each kind and iteration:
 //
-//   phase 0        P x GEN0 (generation 0 of the population) and, when I > 0,
-//                  P x GENMC(0) (generation 1 of the new population, then its
-//                  local search, mc_call 0)
-//   phase k, 1..I  P x MC2(k-1) (local search of the survivors, mc_call
-//                  2(k-1)+1) and, when k < I, P x GENMC(k) (generation k+1,
-//                  local search with mc_call 2k)
+//   GEN0           generation 0: the first survivors
+//   GENMC(i)       generation i + 1, then its local search (mc_call 2i): the new
+//                  population of iteration i, in slots of ring i mod W
+//   MC2(i)         local search of the survivors of iteration i's merge
+//                  (mc_call 2i + 1)
 //
-// The CTA that finishes the last job of a structure's phase runs the phase
-// transition itself -- stable sort of the survivors, then the merge
-// (pyhea/cpp/accelerate.cpp:305-330, :693) -- and appends the next phase's
-// jobs.  With a tolerance, a local search also ends once its f2 is at or
-// below it, and the structure ends once the best f2 after a survivors' sort
-// is (the search of the population generated meanwhile is dropped).
+// A new population depends on nothing but the seed, so W of them (`ahead`) are
+// queued from the start; iteration i's merge waits for population i and for the
+// survivors of iteration i - 1 (two tokens, BatchState::join), and frees
+// population i's slots for population i + W.  So a structure's chain is one long
+// search and I short ones, not I long ones, and its long searches fill the chip.
+// The CTA that finishes the last job of a kind, or brings the second token, runs
+// the transition itself -- stable sort of the survivors, then the merge
+// (pyhea/cpp/accelerate.cpp:305-330, :693) -- and appends the jobs it frees.
+// With a tolerance, a local search also ends once its f2 is at or below it, and
+// the structure ends at the merge that finds the survivors' best f2 at or below
+// it (the population it waited for is dropped); W is then 1, so that no more
+// than that one is searched in vain.
 //
-// Jobs live in ring queues, one per priority level, whose head and tail only
-// grow; a CTA takes the next reserved job of the highest level that has one
-// and waits for the producer's sequence number in the slot.  A ring needs
-// room for the jobs of one phase of every structure at its level (at most
-// 2P each), since a phase is queued only after the previous one finished.
+// Jobs live in ring queues, two per priority level (survivors' jobs before new
+// populations'), whose head and tail only grow; a CTA's first warp looks at all
+// rings at once, takes the next reserved job of the first that has one and waits
+// for the producer's sequence number in the slot.  A ring needs room for the
+// unfinished jobs of its kind of every structure at its level (at most W P each).
 //
 // A launch ends when no structure is active or, for the time slices of the
 // serving loop, at its deadline: CTAs stop taking jobs, and a local search
@@ -71,25 +76,31 @@ struct BatchStruct {
     uint8_t *occ;
     int32_t *cnt;
     double *f2;
-    int32_t *order;    // [2P] slot ids
+    int32_t *order;    // [P (W + 1)] slot ids: the survivors', then each new population's
     int32_t *scratch;  // [2P] sort scratch
-    uint64_t *hist;    // [2P][N] site histograms (SiteHist)
+    uint64_t *hist;    // [P (W + 1)][N] site histograms (SiteHist)
     const uint32_t *nbmask;
     int32_t P, Q, D, I;
     int64_t max_rounds;
     double tol2;  // tolerance on f2 (< 0: none): local searches and the structure end once reached
     int32_t T, layout, level, hbm;
+    int32_t ahead, pad_;  // W: new populations in flight, 1..kBatchAhead
 };
 
 static_assert(sizeof(SearchConst) % 8 == 0 && alignof(SearchConst) >= 8, "SearchConst copied as 8-byte words");
 
+constexpr int kBatchAhead = 4;
+
 struct BatchState {
-    int32_t remaining;  // jobs of the current phase not finished
-    int32_t phase;      // at the end: the iterations run
-    int32_t done;       // 1 once the structure's search ended
-    int32_t pad_;
+    int32_t survivors;          // survivors' jobs (GEN0 or MC2) not finished
+    int32_t left[kBatchAhead];  // jobs of each new population not finished
+    int32_t join[kBatchAhead];  // tokens of the merge of each: 2 once survivors and population are ready
+    int32_t iter;               // iteration of the survivors' jobs (-1: GEN0)
+    int32_t phase;              // at the end: the iterations run
+    int32_t done;               // 1 once the structure's search ended
     unsigned long long tally[3];  // rounds, evals, accepts of this structure
 };
+static_assert(sizeof(BatchState) % 8 == 0, "BatchState copied whole");
 
 constexpr int kBatchLevels = 16;
 
@@ -100,8 +111,11 @@ struct BatchQueue {
     unsigned long long base;  // first slot of this ring in the job array
 };
 
+constexpr int kBatchRings = 2 * kBatchLevels;  // ring 2 l: survivors' jobs of level l; 2 l + 1: new populations'
+static_assert(kBatchRings == 32, "one lane per ring (claim_job)");
+
 struct BatchCtl {
-    BatchQueue q[kBatchLevels];
+    BatchQueue q[kBatchRings];
     unsigned long long stats[4];  // rounds, evals, accepts, finished structures
     int32_t error;                // 1: a wait ran out of time, 2: a ring slot was overwritten
     int32_t active;               // structures seeded and not finished

@@ -2023,7 +2023,7 @@ extern "C" int hea_recount_noalloc(const hea_problem *problem, int32_t count, co
 
 namespace {
 struct BatchLevels {
-    unsigned long long total[kBatchLevels], base[kBatchLevels];
+    unsigned long long total[kBatchRings], base[kBatchRings];
 };
 }  // namespace
 using BatchLevels_ = BatchLevels;
@@ -2072,7 +2072,7 @@ __global__ void batch_reset_kernel(BatchCtl *ctl, BatchJob *jobs, unsigned long 
          i += (unsigned long long)gridDim.x * blockDim.x)
         jobs[i].seq = 0;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        for (int l = 0; l < kBatchLevels; ++l) {
+        for (int l = 0; l < kBatchRings; ++l) {
             ctl->q[l].head = 0;
             ctl->q[l].tail = 0;
             ctl->q[l].cap = lv.total[l] ? lv.total[l] : 1;
@@ -2130,6 +2130,9 @@ int batch_smem_budget(size_t *out, int ctas_per_sm = HEA_BATCH_MIN_BLOCKS)
     return HEA_OK;
 }
 
+// Population memory up to which a batch keeps kBatchAhead new populations of each structure in flight.
+constexpr size_t kBatchAheadBytes = (size_t)6 << 30;
+
 // Launch configuration of a batch: occupancy placement (hbm_all: every
 // structure's occupancy in HBM; otherwise in shared memory where the per-CTA
 // budget of ctas_per_sm CTAs per SM allows) and resident CTAs per SM; then the
@@ -2182,6 +2185,26 @@ int batch_configure(hea_batch *b, int hbm_all, int ctas_per_sm)
 
 extern "C" {
 
+namespace {
+// Population buffers of every structure of a batch with at most `ahead` new populations in flight.
+int batch_populations(hea_batch *b, int ahead)
+{
+    for (BatchStruct &d : b->h_structs) {
+        d.ahead = std::max(1, std::min(ahead, d.I));
+        const size_t slots = (size_t)d.P * (d.ahead + 1), occ_bytes = slots * d.c.occ_stride;
+        const size_t ncount = (size_t)d.c.num_shells * d.c.num_types * d.c.num_types;
+        HEA_TRY(batch_alloc(b, &d.occ, occ_bytes));
+        HEA_TRY(batch_alloc(b, &d.cnt, slots * ncount * sizeof(int32_t)));
+        HEA_TRY(batch_alloc(b, &d.f2, slots * sizeof(double)));
+        HEA_TRY(batch_alloc(b, &d.order, slots * sizeof(int32_t)));
+        HEA_TRY(batch_alloc(b, &d.scratch, 2 * (size_t)d.P * sizeof(int32_t)));
+        HEA_TRY(batch_alloc(b, &d.hist, hist_bytes_of(d.c, (int64_t)slots)));
+        HEA_CUDA(cudaMemset(d.occ, 0, occ_bytes));
+    }
+    return HEA_OK;
+}
+}  // namespace
+
 int hea_batch_create(const hea_problem *problems, const hea_params *params, int32_t count, hea_batch **out)
 {
     if (!out) return fail(HEA_ERR_INVALID, "out is NULL");
@@ -2207,10 +2230,9 @@ int hea_batch_create(const hea_problem *problems, const hea_params *params, int3
             rc = fail(rc, "structure %d: %s", i, m.c_str());
             break;
         }
-        const int P = params[i].num_solutions, slots = 2 * P;
+        const int P = params[i].num_solutions;
         BatchStruct d{};
         d.c = t->c;
-        hist_total += hist_bytes_of(d.c, slots);
         d.nbor = t->nbor;
         d.P = P;
         d.Q = params[i].parallel_task;
@@ -2220,20 +2242,27 @@ int hea_batch_create(const hea_problem *problems, const hea_params *params, int3
         d.tol2 = -1.0;
         d.T = t->T;
         d.layout = batch_layout(t->c, t->S);
-        if ((rc = batch_alloc(b, &d.occ, (size_t)slots * t->c.occ_stride)) != HEA_OK) break;
-        if ((rc = batch_alloc(b, &d.cnt, (size_t)slots * t->ncount * sizeof(int32_t))) != HEA_OK) break;
-        if ((rc = batch_alloc(b, &d.f2, (size_t)slots * sizeof(double))) != HEA_OK) break;
-        if ((rc = batch_alloc(b, &d.order, (size_t)slots * sizeof(int32_t))) != HEA_OK) break;
-        if ((rc = batch_alloc(b, &d.scratch, (size_t)slots * sizeof(int32_t))) != HEA_OK) break;
-        if ((rc = batch_alloc(b, &d.hist, hist_bytes_of(d.c, slots))) != HEA_OK) break;
         d.nbmask = t->nbmask;
-        if (cudaMemset(d.occ, 0, (size_t)slots * t->c.occ_stride) != cudaSuccess) {
-            rc = fail(HEA_ERR_CUDA, "cudaMemset failed");
-            break;
-        }
         b->h_structs.push_back(d);
-        b->total_jobs += d.I > 0 ? (unsigned long long)P * (2 * d.I + 1) : (unsigned long long)P;
+        b->total_jobs += (unsigned long long)P * (2 * d.I + 1);
     }
+    // new populations in flight: as many as kBatchAheadBytes of populations allow, or fewer where the
+    // device has no room for them
+    int ahead = kBatchAhead;
+    for (; rc == HEA_OK && ahead > 1; --ahead) {
+        size_t bytes = 0;
+        for (const BatchStruct &d : b->h_structs)
+            bytes += (hist_bytes_of(d.c, 1) + 2 * (size_t)d.c.num_sites) * d.P * (std::max(1, std::min(ahead, d.I)) + 1);
+        if (bytes <= kBatchAheadBytes) break;
+    }
+    if (rc == HEA_OK) rc = batch_populations(b, ahead);
+    if (rc == HEA_ERR_NOMEM && ahead > 1) {
+        cudaGetLastError();
+        for (void *p : b->buffers) dev_free(p);
+        b->buffers.clear();
+        rc = batch_populations(b, 1);
+    }
+    for (const BatchStruct &d : b->h_structs) hist_total += hist_bytes_of(d.c, 2 * d.P);
     for (BatchStruct &d : b->h_structs) d.c.hist_stream = stream_histograms(hist_bytes_of(d.c, 2 * d.P), hist_total);
     // priority levels: structures ranked by work, largest first
     BatchLevels lv{};
@@ -2248,9 +2277,10 @@ int hea_batch_create(const hea_problem *problems, const hea_params *params, int3
         for (int r = 0; r < count; ++r) {
             BatchStruct &d = b->h_structs[rank[r]];
             d.level = (int)((long long)r * kBatchLevels / count);
-            lv.total[d.level] += d.I > 0 ? (unsigned long long)d.P * (2 * d.I + 1) : (unsigned long long)d.P;
+            lv.total[2 * d.level] += (unsigned long long)d.P * (d.I + 1);  // GEN0 and MC2
+            lv.total[2 * d.level + 1] += (unsigned long long)d.P * d.I;    // GENMC
         }
-        for (int l = 1; l < kBatchLevels; ++l) lv.base[l] = lv.base[l - 1] + lv.total[l - 1];
+        for (int l = 1; l < kBatchRings; ++l) lv.base[l] = lv.base[l - 1] + lv.total[l - 1];
     }
     size_t max_out = 0;
     for (int i = 0; rc == HEA_OK && i < count; ++i)
@@ -2273,11 +2303,15 @@ int hea_batch_create(const hea_problem *problems, const hea_params *params, int3
         if (e == cudaSuccess) e = allow_max_smem(batch_kernel_fn());
         if (e != cudaSuccess) rc = fail(HEA_ERR_CUDA, "batch set-up failed: %s", cudaGetErrorString(e));
     }
-    // Occupancy in HBM by default: with site-histogram scoring a search reads it
-    // only for its draws, and small shared memory leaves room for more CTAs per
-    // SM and a larger L1 (measured faster on the mixed batch; hea_batch_autotune
-    // compares the alternatives on the batch at hand).
-    if (rc == HEA_OK) rc = batch_configure(b, 1, HEA_BATCH_MIN_BLOCKS);
+    // Occupancy staged in shared memory when every structure's fits HEA_BATCH_MIN_BLOCKS CTAs per SM (the
+    // draws' loads then do not go through L1, which three CTAs' rows overflow from some 20 000 sites on),
+    // else in HBM for all: one launch has one shared-memory size, and what it takes is L1 that the
+    // structures in HBM draw through.  Measured, HBM -> staged: eight FCC 20^3 20.3 -> 16.0 ms, eight BCC
+    // 20^3 7.0 -> 6.5 ms; cells of edge 6 to 30 mixed, the largest in HBM either way, 56.5 -> 82.3 ms.
+    // hea_batch_autotune compares the alternatives on the batch at hand.
+    if (rc == HEA_OK) rc = batch_configure(b, 0, HEA_BATCH_MIN_BLOCKS);
+    if (rc == HEA_OK && std::any_of(b->h_structs.begin(), b->h_structs.end(), [](const BatchStruct &d) { return d.hbm; }))
+        rc = batch_configure(b, 1, HEA_BATCH_MIN_BLOCKS);
     if (rc != HEA_OK) {
         delete b;
         return rc;
@@ -2471,6 +2505,7 @@ struct ServerRequest {
     int slot = -1, hbm = 0;
     size_t off = 0, bytes = 0;
     size_t hist_bytes = 0;  // site-histogram bytes of the placed request
+    unsigned long long ring_load = 0;  // ring slots it holds at its level
     double t_submit = 0, t_admit = 0, t_finish = 0, device_ms = 0;
     int iterations = 0;
     unsigned long long tally[3] = {0, 0, 0};
@@ -2498,16 +2533,19 @@ struct ServerRequest {
     }
 };
 
-// Arena bytes of a request: padded table, then 2P occupancy rows, counts,
-// f2, order and sort scratch, each 256-byte aligned.
+constexpr size_t kServerAheadBytes = (size_t)64 << 20;  // arena bytes up to which a request keeps populations ahead
+
+// Arena bytes of a request with `ahead` new populations in flight: padded table,
+// then P (ahead + 1) occupancy rows, counts, f2 and order, and the sort scratch,
+// each 256-byte aligned.
 struct RequestLayout {
     size_t nbor, nbmask, hist, occ, cnt, f2, order, scratch, total;
 };
 
-RequestLayout request_layout(const SearchConst &c, int64_t pad_row, int S, int T, int P)
+RequestLayout request_layout(const SearchConst &c, int64_t pad_row, int S, int T, int P, int ahead)
 {
     RequestLayout L{};
-    const size_t slots = 2 * (size_t)P;
+    const size_t slots = (size_t)P * (ahead + 1);
     size_t o = 0;
     auto take = [&](size_t bytes) {
         const size_t at = o;
@@ -2521,7 +2559,7 @@ RequestLayout request_layout(const SearchConst &c, int64_t pad_row, int S, int T
     L.cnt = take(slots * (size_t)S * T * T * sizeof(int32_t));
     L.f2 = take(slots * sizeof(double));
     L.order = take(slots * sizeof(int32_t));
-    L.scratch = take(slots * sizeof(int32_t));
+    L.scratch = take(2 * (size_t)P * sizeof(int32_t));
     L.total = o;
     return L;
 }
@@ -2640,10 +2678,22 @@ int server_place(hea_server *sv, ServerRequest &r, int slot)
     fill_const(&pb, r.params.seed, c, g);
     const bool implicit = c.lat.L > 0;  // lattice requests: no table in the arena
     const int P = r.params.num_solutions;
-    const RequestLayout L = request_layout(c, implicit ? 0 : g.pad_row, r.S, r.T, P);
-    if (sv->level_load[r.level] + 2ull * P > (unsigned long long)sv->cfg.ring_jobs) return HEA_PENDING;
+    // populations ahead (batch kernel): one with a tolerance, whose later ones may be in vain; else as
+    // many as fill the chip, while the request stays small (kServerAheadBytes) and fits its arena and ring
+    int ahead = 1;
+    RequestLayout L = request_layout(c, implicit ? 0 : g.pad_row, r.S, r.T, P, ahead);
+    while (r.tol2 < 0.0 && ahead < std::min(kBatchAhead, r.params.total_iter) && P * ahead < sv->grid) {
+        const RequestLayout M = request_layout(c, implicit ? 0 : g.pad_row, r.S, r.T, P, ahead + 1);
+        if (M.total > std::min(kServerAheadBytes, (size_t)sv->cfg.arena_bytes) || (ahead + 1ll) * P > sv->cfg.ring_jobs / 8)
+            break;
+        L = M;
+        ++ahead;
+    }
+    const unsigned long long load = 2ull * ahead * P;  // a level's two rings have half of ring_jobs each
+    if (sv->level_load[r.level] + load > (unsigned long long)sv->cfg.ring_jobs) return HEA_PENDING;
     size_t off = 0;
     if (!sv->heap.alloc(L.total, &off)) return HEA_PENDING;
+    r.ring_load = load;
     r.off = off;
     r.bytes = L.total;
     uint8_t *base = sv->arena + off;
@@ -2698,6 +2748,7 @@ int server_place(hea_server *sv, ServerRequest &r, int slot)
     d.I = r.params.total_iter;
     d.max_rounds = r.params.max_rounds > 0 ? r.params.max_rounds : (int64_t)1 << 31;
     d.tol2 = r.tol2;
+    d.ahead = ahead;
     d.T = r.T;
     d.layout = batch_layout(c, r.S);
     d.level = r.level;
@@ -2707,7 +2758,7 @@ int server_place(hea_server *sv, ServerRequest &r, int slot)
                 : 0;
     r.hbm = d.hbm;
     sv->h_structs[slot] = d;
-    sv->level_load[r.level] += 2ull * P;
+    sv->level_load[r.level] += r.ring_load;
     r.slot = slot;
     return HEA_OK;
 }
@@ -2717,7 +2768,7 @@ void server_release(hea_server *sv, ServerRequest &r)
     if (r.slot < 0) return;
     sv->heap.release(r.off, r.bytes);
     sv->hist_placed -= r.hist_bytes;
-    sv->level_load[r.level] -= 2ull * r.params.num_solutions;
+    sv->level_load[r.level] -= r.ring_load;
     sv->slot_req[r.slot] = 0;
     r.slot = -1;
 }
@@ -2892,7 +2943,7 @@ int server_enqueue(hea_server *sv, ServerRequest &&r, const hea_params *params, 
         SearchConst c;
         PadGeom g;
         fill_const(&pb, params->seed, c, g);
-        const RequestLayout L = request_layout(c, c.lat.L ? 0 : g.pad_row, r.S, r.T, params->num_solutions);
+        const RequestLayout L = request_layout(c, c.lat.L ? 0 : g.pad_row, r.S, r.T, params->num_solutions, 1);
         if (L.total > sv->heap.total)
             return fail(HEA_ERR_UNSUPPORTED, "request needs %zu bytes of device memory; the arena holds %zu", L.total,
                         sv->heap.total);
@@ -2950,7 +3001,7 @@ int hea_server_create(const hea_server_config *config, hea_server **out)
     if (rc == HEA_OK) rc = sv->alloc(&sv->arena, (size_t)cfg.arena_bytes);
     if (rc == HEA_OK) rc = sv->alloc(&sv->d_structs, sizeof(BatchStruct) * M);
     if (rc == HEA_OK) rc = sv->alloc(&sv->d_states, sizeof(BatchState) * M);
-    if (rc == HEA_OK) rc = sv->alloc(&sv->d_jobs, sizeof(BatchJob) * (size_t)cfg.ring_jobs * kBatchLevels);
+    if (rc == HEA_OK) rc = sv->alloc(&sv->d_jobs, sizeof(BatchJob) * (size_t)(cfg.ring_jobs / 2) * kBatchRings);
     if (rc == HEA_OK) rc = sv->alloc(&sv->d_ctl, sizeof(BatchCtl));
     if (rc == HEA_OK) rc = sv->alloc(&sv->d_finish, sizeof(unsigned long long) * M);
     if (rc == HEA_OK) rc = sv->alloc(&sv->d_list, sizeof(int32_t) * M);
@@ -2984,12 +3035,12 @@ int hea_server_create(const hea_server_config *config, hea_server **out)
         if (e == cudaSuccess) e = cudaMemsetAsync(sv->d_finish, 0, sizeof(unsigned long long) * M, sv->stream);
         if (e == cudaSuccess) {
             BatchLevels lv{};
-            for (int l = 0; l < kBatchLevels; ++l) {
-                lv.total[l] = (unsigned long long)cfg.ring_jobs;
-                lv.base[l] = (unsigned long long)l * cfg.ring_jobs;
+            for (int l = 0; l < kBatchRings; ++l) {
+                lv.total[l] = (unsigned long long)(cfg.ring_jobs / 2);
+                lv.base[l] = (unsigned long long)l * (cfg.ring_jobs / 2);
             }
             batch_reset_kernel<<<64, 256, 0, sv->stream>>>(sv->d_ctl, sv->d_jobs,
-                                                          (unsigned long long)cfg.ring_jobs * kBatchLevels, lv,
+                                                          (unsigned long long)(cfg.ring_jobs / 2) * kBatchRings, lv,
                                                           (unsigned long long)(cfg.wait_limit_ms * 1e6));
             e = cudaGetLastError();
         }

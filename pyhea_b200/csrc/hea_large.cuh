@@ -209,6 +209,7 @@ __global__ void __launch_bounds__(512, 2) mc_large_kernel(const __grid_constant_
                     cta_rec[round & 1].lo = cta_rec[round & 1].hi = kNoSwap;
             }
         }
+        __syncwarp();
         cluster.sync();
         // every warp reduces the cluster's records
         float lo = kNoSwap, hi = kNoSwap;
@@ -230,6 +231,7 @@ __global__ void __launch_bounds__(512, 2) mc_large_kernel(const __grid_constant_
             // the cluster's next proposals read the histograms and species bits rank 0 updated: rank 0
             // arrives with release semantics, the others (whose accept work stays in their own shared
             // memory, ordered by the block barrier) relaxed, every thread waits with acquire semantics.  Measured: 4 % per round.
+            __syncwarp();
             __syncthreads();  // this CTA's warps read the new counts and table
             if (rank == 0)
                 __cluster_barrier_arrive();

@@ -635,7 +635,8 @@ struct HistEntry {
 template <class H>
 __device__ __forceinline__ int hist_field(const HistEntry<H::W> &e, int k, int t)  // t < T - 1
 {
-    return (int)((uint32_t)(e.w[H::word(k, t)] >> H::shift(k, t)) & ((1u << H::width(k)) - 1u));
+    const uint64_t w = H::W == 1 ? e.w[0] : H::word(k, t) ? e.w[H::W - 1] : e.w[0];  // no indexed array (k, t at run time)
+    return (int)((uint32_t)(w >> H::shift(k, t)) & ((1u << H::width(k)) - 1u));
 }
 template <class H, int T>
 __device__ __forceinline__ uint64_t hist_unit(int k, int t)  // one neighbour of species t in shell k
@@ -885,20 +886,22 @@ __device__ __forceinline__ double exact_delta(const SearchConst &c, const int32_
     return D;
 }
 
-// The same by one lane alone, each of the calling lanes with its own proposal.
+// The same by one lane alone, each of the active lanes with its own proposal.
+// Rolled loops: it is rare, and the search loop's code stays small.  Inlined, so
+// that its registers are the search loop's (as a call it cost spills there).
 template <int T, class L, int W>
-__device__ __noinline__ double exact_delta_lane(const SearchConst &c, const int32_t *cnt, int ab, HistEntry<W> p,
-                                                HistEntry<W> q)
+__device__ __forceinline__ double exact_delta_lane(const SearchConst &c, const int32_t *cnt, int ab,
+                                                   const HistEntry<W> &p, const HistEntry<W> &q)
 {
     constexpr int S = L::S;
     using H = SiteHist<T, S, L::kImplicit>;
     const int a = ab & 0xFF, b = ab >> 8;
     double D = 0.0;
-#pragma unroll
+#pragma unroll 1
     for (int k = 0; k < S; ++k) {
         const double *R = c.R + k * T * T, *E = c.E + k * T * T, w = c.w[k];
         int rest = 0, v = 0;
-#pragma unroll
+#pragma unroll 1
         for (int t = 0; t < T; ++t) {
             const int u = t < T - 1 ? hist_field<H>(q, k, t) - hist_field<H>(p, k, t) : -rest;
             rest += u;
@@ -1072,7 +1075,9 @@ __device__ __forceinline__ bool draw_pair_by(const SearchConst &c, uint32_t stre
 // All attempts of the first call at once -- the species of every attempt's sites
 // in one round trip to shared memory, no branch -- then the calls after it.  A
 // warp needs 3 of 4 attempts on average before its last lane has a pair, so the
-// loop's dependent loads cost more than the loads left unused.
+// loop's dependent loads cost more than the loads left unused (batch of FCC
+// 20^3 structures, occupancy in shared memory: 17.4 -> 16.0 ms; in HBM, through
+// L1: no difference).
 template <bool k16>
 __device__ __forceinline__ bool draw_pair_at_once(const SearchConst &c, uint32_t stream, uint32_t round, uint32_t task,
                                                   const uint8_t *occ, uint32_t &s1, uint32_t &s2)
@@ -1099,15 +1104,12 @@ __device__ __forceinline__ bool draw_pair_at_once(const SearchConst &c, uint32_t
     return ok;
 }
 
-// Species from the occupancy: all first attempts at once where it lies in shared memory.
-template <bool kShared>
+// Species from the occupancy.
 __device__ __forceinline__ bool draw_pair(const SearchConst &c, uint32_t stream, uint32_t round, uint32_t task,
                                           const uint8_t *occ, uint32_t &s1, uint32_t &s2)
 {
-    if constexpr (kShared)
-        return c.draw16 ? draw_pair_at_once<true>(c, stream, round, task, occ, s1, s2)
-                        : draw_pair_at_once<false>(c, stream, round, task, occ, s1, s2);
-    return draw_pair_by(c, stream, round, task, [occ](uint32_t u, uint32_t v) { return occ[u] != occ[v]; }, s1, s2);
+    return c.draw16 ? draw_pair_at_once<true>(c, stream, round, task, occ, s1, s2)
+                    : draw_pair_at_once<false>(c, stream, round, task, occ, s1, s2);
 }
 
 // Species from the site histograms' top bits: for an occupancy in HBM this
@@ -1358,8 +1360,22 @@ __device__ __forceinline__ void keep_best(const SearchConst &c, const int32_t *c
         if (cand & (cand - 1)) win = resolve<T, L>(c, cnt, (cand >> lane) & 1u, r.task, r.ab, r.p, r.q);
         if (lane == win) {
             bool take = !more || r.hi < mine.lo;
-            if (!take && r.lo <= mine.hi)  // an earlier pass's best too near to tell; on equal D it has the lower task
-                take = exact_delta_lane<T, L>(c, cnt, r.ab, r.p, r.q) < exact_delta_lane<T, L>(c, cnt, mine.ab, mine.p, mine.q);
+            if (!take && r.lo <= mine.hi) {  // an earlier pass's best too near to tell; on equal D it has the lower task
+                double before = 0.0, D = 0.0;
+#pragma unroll 1
+                for (int x = 0; x < 2; ++x) {
+                    auto p = r.p, q = r.q;
+                    int ab = r.ab;
+                    if (x == 0) {
+                        p = mine.p;
+                        q = mine.q;
+                        ab = mine.ab;
+                    }
+                    before = D;
+                    D = exact_delta_lane<T, L>(c, cnt, ab, p, q);
+                }
+                take = D < before;
+            }
             if (take) mine = r;
         }
     }
@@ -1428,10 +1444,10 @@ __device__ __forceinline__ void search_setup(const SearchConst &c, const int32_t
 // Rounds of the local search on the staged state: occupancy occ, counts in
 // buffer 0 of cnt2, the delta table tab (search_setup), running f2 `cur`.
 // Every thread returns the same tally; evals is this thread's count.  No
-// barrier at entry.  occ is in shared memory (kShared) or global memory.  The
+// barrier at entry.  occ is in shared or global memory.  The
 // draws read the species from occ; proposals are scored from the
 // site histograms `hist`, which an accept updates.
-template <int T, class L, bool kShared, bool kYield = false>
+template <int T, class L, bool kYield = false>
 __device__ __forceinline__ McTally mc_rounds(const SearchConst &c, const int4 *__restrict__ nbor, uint8_t *occ,
                                              int32_t *cnt2, const DeltaTab<T, L::S> tab, void *records, uint32_t stream,
                                              double cur, int tasks, int depth, int64_t max_rounds, McTrace tr,
@@ -1458,7 +1474,7 @@ __device__ __forceinline__ McTally mc_rounds(const SearchConst &c, const int4 *_
         for (int q0 = warp * 32; q0 < tasks; q0 += blockDim.x) {
             const int q = q0 + lane;
             uint32_t s1 = 0, s2 = 0;  // a lane without a pair scores site 0 with itself and drops the result
-            const bool ok = q < tasks && draw_pair<kShared>(c, stream, (uint32_t)round, (uint32_t)q, occ, s1, s2);
+            const bool ok = q < tasks && draw_pair(c, stream, (uint32_t)round, (uint32_t)q, occ, s1, s2);
             __syncwarp();  // lanes that needed more draws rejoin before scoring
             undrawn += q < tasks && !ok;
             Record r;
@@ -1477,6 +1493,7 @@ __device__ __forceinline__ McTally mc_rounds(const SearchConst &c, const int4 *_
         }
         // the stop decision travels in warp 0's record (read by all after the barrier)
         if (kYield && tid == 0) rr[0].stop = (rs.deadline_ns && global_ns() >= rs.deadline_ns) ? 1 : 0;
+        __syncwarp();
         __syncthreads();
         const bool stop = kYield && rr[0].stop != 0;
         // every warp reduces the records of all warps
@@ -1497,6 +1514,7 @@ __device__ __forceinline__ McTally mc_rounds(const SearchConst &c, const int4 *_
                 const double D = exact_delta<T, L>(c, cold, a, b, w.p, w.q);
                 if (lane == 0) *tab.accepted() = D;
             }
+            __syncwarp();
             __syncthreads();  // next round's proposals read the new table and histograms
             buf ^= 1;
             if (track) cur = __dadd_rn(cur, *tab.accepted());
@@ -1591,7 +1609,7 @@ __global__ void __launch_bounds__(512, HEA_MC_MIN_BLOCKS) mc_kernel(const __grid
         tr.counts = g.trace_counts ? g.trace_counts + (size_t)blockIdx.x * g.trace_cap * NC : nullptr;
         tr.cap = g.trace_cap;
     }
-    const McTally t = mc_rounds<T, L, true>(c, g.nbor, occ, cnt2, tab, rec, stream, g.f2[slot], g.tasks, g.depth,
+    const McTally t = mc_rounds<T, L>(c, g.nbor, occ, cnt2, tab, rec, stream, g.f2[slot], g.tasks, g.depth,
                                       g.max_rounds, tr, McResume{0, 0, 0ull, -1.0},
                                       g.hist + (size_t)slot * c.num_sites * hist_words(T, S, L::kImplicit),
                                       g.nbmask);

@@ -76,3 +76,41 @@ def test_after_release_of_cached_memory():
     for _ in range(2):
         same(hb.search(gp, 3, 3, 24, 3, seed=4), op.hcs(4, 3, 3, 24, 3))
         hb.lib.hea_release_cached_memory()
+
+
+@pytest.mark.parametrize("iters", [0, 1, 3, 4, 5, 11])
+def test_batch_populations_ahead(iters):
+    """Iterations around the populations a batch keeps in flight; the first structure has two more."""
+    cases = [case(20 + i, species=(18, 18, 18)) for i in range(4)]
+    its = [iters + 2 if i == 0 else iters for i in range(4)]
+    b = hb.Batch([gp for gp, _ in cases],
+                 [dict(num_solutions=3 + i, total_iter=its[i], parallel_task=24, converge_depth=3) for i in range(4)])
+    for seeds in ((5, 6, 7, 8), (15, 6, 17, 8)):
+        b.run(seeds)
+        for i, (_, op) in enumerate(cases):
+            same(b.read(i), op.hcs(seeds[i], 3 + i, its[i], 24, 3))
+    b.close()
+
+
+@pytest.mark.parametrize("tasks", [16, 32, 37, 64, 100, 256, 300])
+def test_batch_counts_each_job_once(tasks):
+    """Rounds, evaluations and accepts for task counts that leave warps of a CTA idle or part full."""
+    gp, op = case(3, lattice=L.BCC, cell=5, species=(100, 75, 75))
+    b = hb.Batch([gp], [dict(num_solutions=7, total_iter=2, parallel_task=tasks, converge_depth=4)])
+    b.run([9])
+    want = op.hcs(9, 7, 2, tasks, 4)
+    same(b.read(0), want)
+    assert [int(v) for v in b.tallies()[0]] == [want[2]["rounds"], want[2]["evals"], want[2]["accepts"]]
+    b.close()
+
+
+def test_served_requests_with_populations_ahead():
+    cases = [case(40 + i) for i in range(5)]
+    srv = hb.Server(slice_ms=0.2)
+    prm = [dict(num_solutions=3 + i, total_iter=2 * i + 1, parallel_task=24, converge_depth=3, seed=60 + i)
+           for i in range(5)]
+    ids = [srv.submit(gp, q) for (gp, _), q in zip(cases, prm)]
+    srv.drain()
+    for rid, (_, op), q in zip(ids, cases, prm):
+        same(srv.result(rid), op.hcs(q["seed"], q["num_solutions"], q["total_iter"], 24, 3))
+    srv.close()

@@ -2059,7 +2059,7 @@ extern "C" int hea_recount_noalloc(const hea_problem *problem, int32_t count, co
 }
 
 // ---------------------------------------------------------------------------
-// Batched search: many structures in one persistent kernel (hea_batch.cuh)
+// Batched search: many structures in one persistent kernel (hea_batch.h)
 // ---------------------------------------------------------------------------
 #include "hea_batch.h"
 
@@ -2480,7 +2480,7 @@ void hea_batch_destroy(hea_batch *b) { delete b; }
 }  // extern "C"
 
 // ---------------------------------------------------------------------------
-// Serving loop (hea_server_*): the job engine of hea_batch.cuh run in time
+// Serving loop (hea_server_*): the job engine of hea_batch.h run in time
 // slices.  Between slices the host admits queued requests (tables built or
 // uploaded into a device arena, phase-0 jobs seeded) and collects finished
 // ones; requests still running keep their state on the device.

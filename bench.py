@@ -77,17 +77,17 @@ HBM_FALLBACK_GBS = 6650.0
 #   dram_read  dram__bytes_read.sum                           -> roofline.dram_random (batched)
 # mc_kernel<5, ImplicitShells<3>> (the plain structure's table is recognised as a BCC lattice's): the
 # first local-search launch of `python bench.py --case plain --iters 1` (203.72 M evaluations):
-# 69.81 MB + 92.28 MB DRAM, 428.96 M L2 sectors, 3.9814 G warp instructions.  batch_kernel: the launch
+# 37.02 MB + 4.27 MB DRAM, 418.07 M L2 sectors, 3.6224 G warp instructions.  batch_kernel: the launch
 # of `python bench.py --case batch --count 64 --iters 10`, the bench's batch configuration (6268.46 M
-# evaluations, lattice tables recognised): 1189.72 GB + 81.32 GB DRAM, 68.43 G L2 sectors, 178.51 G
+# evaluations, lattice tables recognised): 842.36 GB + 57.09 GB DRAM, 56.92 G L2 sectors, 166.75 G
 # warp instructions.  dram_random_probe_kernel (hea_dram_random_probe over 4 GiB, 77.59 M
 # random 16-byte loads): 9.833 GB DRAM read, i.e. 126.7 B per load (each load fetches a 128-byte line).
 KERNEL_COUNTERS = {
-    "plain_gpu": {"dram": (69.81e6 + 92.28e6) / 203.72e6, "l2": 428.96e6 * 32.0 / 203.72e6,
-                  "inst": 3.9814e9 / 203.72e6,
+    "plain_gpu": {"dram": (37.02e6 + 4.27e6) / 203.72e6, "l2": 418.07e6 * 32.0 / 203.72e6,
+                  "inst": 3.6224e9 / 203.72e6,
                   "capture": "mc_kernel, first local-search launch of bench.py --case plain --iters 1"},
-    "batched": {"dram": (1189.72e9 + 81.32e9) / 6268.46e6, "l2": 68.43e9 * 32.0 / 6268.46e6,
-                "inst": 178.51e9 / 6268.46e6, "dram_read": 1189.72e9 / 6268.46e6,
+    "batched": {"dram": (842.36e9 + 57.09e9) / 6268.46e6, "l2": 56.92e9 * 32.0 / 6268.46e6,
+                "inst": 166.75e9 / 6268.46e6, "dram_read": 842.36e9 / 6268.46e6,
                 "capture": "batch_kernel, bench.py --case batch --count 64 --iters 10"},
 }
 DRAM_BYTES_PER_RANDOM_LOAD = 9.833e9 / 77.594624e6

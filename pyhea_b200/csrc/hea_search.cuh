@@ -1386,7 +1386,9 @@ __device__ __forceinline__ void keep_best(const SearchConst &c, const int32_t *c
         int win = __ffs(cand) - 1;
         if (cand & (cand - 1)) win = resolve<T, L>(c, cnt, (cand >> lane) & 1u, least < 0.0f, r.task, r.ab, r.p, r.q);
         if (lane == win) {
-            bool take = !more || r.hi < mine.lo;
+            // an empty record (lo = kNoSwap: no pass before found a D < 0) has no proposal to compare with, and
+            // where every proposal is exact (screen_floor) its hi equals theirs
+            bool take = !more || mine.lo == kNoSwap || r.hi < mine.lo;
             if (!take && r.lo <= mine.hi) {  // an earlier pass's best too near to tell; on equal D it has the lower task
                 double before = 0.0, D = 0.0;
 #pragma unroll 1

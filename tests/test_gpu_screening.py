@@ -3,7 +3,8 @@ oracle bit for bit where the screening's choices are hardest -- many equal D's
 (two species, one shell), a species of a single atom, targets already met,
 weights or targets outside FP32's range, six species in three shells (both
 histogram widths) -- and where a round takes several passes (CTAs smaller than
-the round, on one CTA and on a cluster, in both draw modes)."""
+the round, on one CTA and on a cluster, in both draw modes), with and without
+the screening."""
 import numpy as np
 import pytest
 
@@ -74,3 +75,38 @@ def test_passes_on_a_cluster(cell, tasks):
     n = L.num_sites(L.FCC, cell)
     gp, op = problems(L.FCC, cell, [n // 4] * 4, 3, L.SHELLS_FCC_TRUE3, seed=1)
     same(gp, op, 2, 1, tasks, 3, seed=5, max_rounds=25, hbm_occupancy=True)
+
+
+OUTSIDE = [
+    ((64, 64, 64, 64), 3, [1e-300, 1.0, 1e300], 1.0),
+    ((64, 64, 64, 64), 3, None, 1e9),
+    ((100, 100, 55, 1), 2, None, 1e8),
+    ((128, 128), 1, None, 1e9),
+    ((60, 50, 50, 40, 30, 26), 3, [1e-300, 1.0, 1e300], 1.0),
+]
+
+
+@pytest.mark.parametrize("species,shells,weight,scale", OUTSIDE)
+@pytest.mark.parametrize("tasks,hbm", [(513, False), (600, False), (1100, False), (4200, True), (8200, True)])
+def test_passes_with_every_proposal_exact(species, shells, weight, scale, tasks, hbm):
+    """Beyond FP32's range no interval tells an empty record from a proposal: passes after one that
+    improved nothing (most of a survivors' search), on one CTA and on clusters, to convergence or
+    some rounds past it."""
+    gp, op = problems(L.FCC, 4, species, shells, seed=len(species), weight=weight, scale=scale)
+    same(gp, op, 2, 2, tasks, 4, seed=tasks, max_rounds=40 if tasks > 2000 else 150, hbm_occupancy=hbm)
+
+
+@pytest.mark.parametrize("species,shells,weight,scale", OUTSIDE)
+def test_batch_passes_with_every_proposal_exact(species, shells, weight, scale):
+    cases = [problems(L.FCC, 4, species, shells, seed=i, weight=weight, scale=scale) for i in range(3)]
+    tasks = (257, 300, 700)
+    b = hb.Batch([gp for gp, _ in cases],
+                 [dict(num_solutions=3, total_iter=2, parallel_task=t, converge_depth=4, max_rounds=150) for t in tasks])
+    for seeds in ((5, 6, 7), (8, 9, 10)):
+        b.run(seeds)
+        for i, (_, op) in enumerate(cases):
+            wocc, wf2, _ = op.hcs(seeds[i], 3, 2, tasks[i], 4, max_rounds=150)
+            occ, fit = b.read(i)[:2]
+            np.testing.assert_array_equal(occ, wocc)
+            np.testing.assert_array_equal(fit, np.sqrt(wf2))
+    b.close()

@@ -2297,12 +2297,14 @@ int hea_batch_create(const hea_problem *problems, const hea_params *params, int3
             bytes += (hist_bytes_of(d.c, 1) + 2 * (size_t)d.c.num_sites) * d.P * (std::max(1, std::min(ahead, d.I)) + 1);
         if (bytes <= kBatchAheadBytes) break;
     }
-    if (rc == HEA_OK) rc = batch_populations(b, ahead);
-    if (rc == HEA_ERR_NOMEM && ahead > 1) {
-        cudaGetLastError();
-        for (void *p : b->buffers) dev_free(p);
-        b->buffers.clear();
-        rc = batch_populations(b, 1);
+    if (rc == HEA_OK) {
+        rc = batch_populations(b, ahead);
+        if (rc == HEA_ERR_NOMEM && ahead > 1) {
+            cudaGetLastError();
+            for (void *p : b->buffers) dev_free(p);
+            b->buffers.clear();
+            rc = batch_populations(b, 1);
+        }
     }
     for (const BatchStruct &d : b->h_structs) hist_total += hist_bytes_of(d.c, 2 * d.P);
     for (BatchStruct &d : b->h_structs) d.c.hist_stream = stream_histograms(hist_bytes_of(d.c, 2 * d.P), hist_total);

@@ -40,6 +40,7 @@ __device__ __forceinline__ void enqueue_jobs(BatchJob *jobs, BatchCtl *ctl, int 
 {
     BatchQueue &q = ctl->q[job_ring(level, kind)];
     if (threadIdx.x == 0) *first_sh = atomicAdd(&q.tail, (unsigned long long)n);
+    __syncwarp();
     __syncthreads();
     const unsigned long long first = *first_sh;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -256,7 +257,22 @@ __device__ __forceinline__ JobEnd batch_dispatch_t(const SearchConst &c, const B
 }
 
 // The persistent kernel: CTAs take jobs until no structure is active or the
-// launch's deadline has passed.  Dynamic shared memory: occupancy of the
+// launch's deadline has passed.
+//
+// Barriers.  Every path through the loop body meets the same barriers in every
+// warp: what decides a path (stop, last, merge, finished) is the same value in
+// all threads, from a barrier or from shared memory behind one.  Shared values
+// are written by thread 0 before the barrier that publishes them and not again
+// until the CTA has met another one behind their last read: job, merge, behind
+// (read behind the barrier on `last`; the next job's barriers follow), first
+// (enqueue_jobs ends with one), c.  Block barriers are instructions of whole
+// warps, so where thread 0 works alone (a wait for a producer, a transition's
+// counts) its warp comes together first (__syncwarp): lanes that reached the
+// barrier ahead of it would count their warp as arrived, and the other warps
+// would go on with the job that stood there before.  That would explain what an
+// earlier form without it, with a plain barrier and a shared stop flag, once
+// did (other warps took the old job again); the form is not run any more, so it
+// is an explanation and not a finding.  Dynamic shared memory: occupancy of the
 // largest shared-memory structure + 16 + per-warp counts + swap records; the
 // job's constants (1.9 KB) are copied to static shared memory.
 __global__ void __launch_bounds__(HEA_BATCH_THREADS, HEA_BATCH_MIN_BLOCKS)
@@ -303,9 +319,8 @@ __global__ void __launch_bounds__(HEA_BATCH_THREADS, HEA_BATCH_MIN_BLOCKS)
                 }
             }
         }
-        // A barrier that carries thread 0's answer (not a plain one and a shared flag: between that and
-        // the barrier that ends the loop body only the first warp works, and the other warps were seen to
-        // run the old job again).
+        // Thread 0's answer travels in the barrier, which needs no shared flag.
+        __syncwarp();
         if (__syncthreads_or(threadIdx.x == 0 && stop)) break;
         // this job's structure: read-only while it is active
         const BatchStruct &d = structs[job.structure];
@@ -345,6 +360,7 @@ __global__ void __launch_bounds__(HEA_BATCH_THREADS, HEA_BATCH_MIN_BLOCKS)
                 }
             }
         }
+        __syncwarp();
         if (!__syncthreads_or(threadIdx.x == 0 && last)) continue;
         bool finished = false;
         if (!population) {
@@ -358,6 +374,7 @@ __global__ void __launch_bounds__(HEA_BATCH_THREADS, HEA_BATCH_MIN_BLOCKS)
                 if (atomicAdd(&st.join[k % d.ahead], 1) == 1) merge = k;
             }
             if (finished && threadIdx.x == 0) st.phase = k;
+            __syncwarp();
             __syncthreads();
         }
         const int it = merge;
@@ -367,6 +384,7 @@ __global__ void __launch_bounds__(HEA_BATCH_THREADS, HEA_BATCH_MIN_BLOCKS)
             if (it > 0 && d.tol2 >= 0.0 && __ldcg(d.f2 + __ldcg(d.order)) <= d.tol2) {
                 finished = true;  // tolerance reached
                 if (threadIdx.x == 0) st.phase = it;
+                __syncwarp();
             } else {
                 block_stable_sort(d.order, P, d.order + (size_t)P * (it % d.ahead + 1), P, d.f2, d.scratch);
             }
@@ -379,6 +397,7 @@ __global__ void __launch_bounds__(HEA_BATCH_THREADS, HEA_BATCH_MIN_BLOCKS)
                 atomicAdd(&ctl->stats[3], 1ull);
                 atomicSub(&ctl->active, 1);
             }
+            __syncwarp();
             __syncthreads();
             continue;
         }
@@ -390,6 +409,7 @@ __global__ void __launch_bounds__(HEA_BATCH_THREADS, HEA_BATCH_MIN_BLOCKS)
             if (more) st.left[it % d.ahead] = P;
             __threadfence();
         }
+        __syncwarp();
         __syncthreads();
         enqueue_jobs(jobs, ctl, d.level, s, kJobMc2, it, P, &first);
         if (more) enqueue_jobs(jobs, ctl, d.level, s, kJobGenMc, it + d.ahead, P, &first);

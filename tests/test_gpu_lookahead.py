@@ -114,3 +114,18 @@ def test_served_requests_with_populations_ahead():
     for rid, (_, op), q in zip(ids, cases, prm):
         same(srv.result(rid), op.hcs(q["seed"], q["num_solutions"], q["total_iter"], 24, 3))
     srv.close()
+
+
+@pytest.mark.parametrize("tasks", [16, 64, 300])
+def test_batch_counts_each_job_once_in_many_runs(tasks):
+    """Several structures with short jobs: CTAs of every structure take and wait for jobs at once, and
+    each run's tallies are the oracle's."""
+    cases = [case(70 + i, cell=3 + i % 3, species=[(20, 17, 17), (48, 40, 40), (100, 75, 75)][i % 3]) for i in range(6)]
+    b = hb.Batch([gp for gp, _ in cases],
+                 [dict(num_solutions=40, total_iter=6, parallel_task=tasks, converge_depth=2)] * len(cases))
+    want = [op.hcs(9 + i, 40, 6, tasks, 2)[2] for i, (_, op) in enumerate(cases)]
+    want = [[w["rounds"], w["evals"], w["accepts"]] for w in want]
+    for _ in range(30):
+        b.run([9 + i for i in range(len(cases))])
+        np.testing.assert_array_equal(b.tallies(), want)
+    b.close()

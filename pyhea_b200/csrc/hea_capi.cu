@@ -1357,13 +1357,13 @@ int plan_search(hea_plan *pl, hea_stats *stats)
 // candidate's rate is its best pass (evaluations per millisecond).  A smaller
 // CTA replaces the default only when its rate is above the default's by more
 // than kTuneMargin, so timing noise cannot trade the default for a near tie.
-// Picks are cached per device and shape for the life of the process.
+// Picks are cached per device and shape for the life of the process; the shape
+// includes what the best size depends on beside the structure: neighbour form,
+// populations in flight and the default they give.
 struct TuneKey {
-    int dev, N, T, S, row4, Q, P;
-    bool operator<(const TuneKey &o) const
-    {
-        return std::tie(dev, N, T, S, row4, Q, P) < std::tie(o.dev, o.N, o.T, o.S, o.row4, o.Q, o.P);
-    }
+    int dev, N, T, S, row4, lattice, Q, P, ahead, standard;
+    auto fields() const { return std::tie(dev, N, T, S, row4, lattice, Q, P, ahead, standard); }
+    bool operator<(const TuneKey &o) const { return fields() < o.fields(); }
 };
 std::mutex g_tune_mu;
 std::map<TuneKey, int> g_tune;
@@ -1379,7 +1379,8 @@ int plan_autotune(hea_plan *pl, bool measure)
     const SearchConst &c = pl->dt.c;
     int dev = 0;
     HEA_CUDA(cudaGetDevice(&dev));
-    const TuneKey key{dev, c.num_sites, pl->dt.T, pl->dt.S, c.row4, pl->prm.parallel_task, pl->P};
+    const TuneKey key{dev, c.num_sites, pl->dt.T, pl->dt.S, c.row4, c.lat.L > 0, pl->prm.parallel_task, pl->P,
+                      (int)pl->ahead.size(), pl->mc_block};
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tune.find(key);

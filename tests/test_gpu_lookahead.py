@@ -49,6 +49,28 @@ def test_plan_runs_again():
     plan.close()
 
 
+def test_a_tuned_size_is_kept_for_plans_with_as_much_in_flight():
+    """The size tuned for one iteration (64 searches at once) is not taken by a plan of sixteen, whose
+    default is smaller CTAs, and the other way round; both give the same search."""
+    st = W.small_case(lattice=L.BCC, cell=10, species=(700, 650, 650), shells=3, seed=1)
+    pb = st.problem()
+    default = {}
+    for iters in (1, 16):
+        with_default = hb.Plan(pb, 64, iters, 512, 2)
+        default[iters] = with_default.local_search_block
+        with_default.close()
+    assert default[1] == 512 and default[16] == 256
+    hb.Plan(pb, 64, 1, 512, 2, autotune=True).close()
+    plan = hb.Plan(pb, 64, 16, 512, 2)
+    assert plan.local_search_block == default[16]
+    hb.Plan(pb, 64, 16, 512, 2, autotune=True).close()
+    one = hb.Plan(pb, 64, 1, 512, 2, autotune=True)
+    again = hb.Plan(pb, 64, 1, 512, 2)
+    assert again.local_search_block == one.local_search_block
+    for p in (plan, one, again):
+        p.close()
+
+
 def test_threads_share_the_stream_cache():
     gp, op = case(9)
     want = {s: op.hcs(s, 3, 4, 24, 3) for s in range(6)}

@@ -71,6 +71,20 @@ def test_a_tuned_size_is_kept_for_plans_with_as_much_in_flight():
         p.close()
 
 
+@pytest.mark.parametrize("P,iters,tasks", [(5, 1, 300), (5, 0, 300), (40, 18, 512), (75, 9, 600), (3, 2, 130)])
+def test_tuned_plans_search_the_same(P, iters, tasks):
+    """Other sizes than the default are tried in the plan's own slots, whatever its iterations."""
+    gp, op = case(31)
+    plan = hb.Plan(gp, P, iters, tasks, 2, autotune=True)
+    passes = -(-tasks // 256)
+    whole, equal = min(512, -(-tasks // 32) * 32), -(-(-(-tasks // passes)) // 32) * 32  # one pass; equal passes
+    assert plan.local_search_block in {whole, equal, 256, 128}
+    for seed in (3, 4):
+        plan.run(seed)
+        same(plan.read(), op.hcs(seed, P, iters, tasks, 2))
+    plan.close()
+
+
 def test_threads_share_the_stream_cache():
     gp, op = case(9)
     want = {s: op.hcs(s, 3, 4, 24, 3) for s in range(6)}

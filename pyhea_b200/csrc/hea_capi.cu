@@ -2724,20 +2724,30 @@ int server_place(hea_server *sv, ServerRequest &r, int slot)
     const bool implicit = c.lat.L > 0;  // lattice requests: no table in the arena
     const int P = r.params.num_solutions;
     // populations ahead (batch kernel): one with a tolerance, whose later ones may be in vain; else as
-    // many as fill the chip, while the request stays small (kServerAheadBytes) and fits its arena and ring
+    // many as fill the chip, while the request stays small (kServerAheadBytes) and leaves room to those
+    // after it: a quarter of the arena and half of its level's ring
     int ahead = 1;
+    unsigned long long load = 2ull * P;  // a level's two rings have half of ring_jobs each
     RequestLayout L = request_layout(c, implicit ? 0 : g.pad_row, r.S, r.T, P, ahead);
     while (r.tol2 < 0.0 && ahead < std::min(kBatchAhead, r.params.total_iter) && P * ahead < sv->grid) {
         const RequestLayout M = request_layout(c, implicit ? 0 : g.pad_row, r.S, r.T, P, ahead + 1);
-        if (M.total > std::min(kServerAheadBytes, (size_t)sv->cfg.arena_bytes) || (ahead + 1ll) * P > sv->cfg.ring_jobs / 8)
+        const unsigned long long more = load + 2ull * P;
+        if (M.total > kServerAheadBytes || M.total + sv->heap.total / 4 > sv->heap.free_bytes ||
+            more > (unsigned long long)sv->cfg.ring_jobs / 4 ||
+            sv->level_load[r.level] + more > (unsigned long long)sv->cfg.ring_jobs / 2)
             break;
         L = M;
+        load = more;
         ++ahead;
     }
-    const unsigned long long load = 2ull * ahead * P;  // a level's two rings have half of ring_jobs each
     if (sv->level_load[r.level] + load > (unsigned long long)sv->cfg.ring_jobs) return HEA_PENDING;
     size_t off = 0;
-    if (!sv->heap.alloc(L.total, &off)) return HEA_PENDING;
+    while (!sv->heap.alloc(L.total, &off)) {  // free memory in smaller pieces: one population may fit
+        if (ahead == 1) return HEA_PENDING;
+        ahead = 1;
+        load = 2ull * P;
+        L = request_layout(c, implicit ? 0 : g.pad_row, r.S, r.T, P, ahead);
+    }
     r.ring_load = load;
     r.off = off;
     r.bytes = L.total;

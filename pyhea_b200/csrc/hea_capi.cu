@@ -2354,9 +2354,14 @@ int hea_batch_create(const hea_problem *problems, const hea_params *params, int3
     // structures in HBM draw through.  Measured, HBM -> staged: eight FCC 20^3 20.3 -> 16.0 ms, eight BCC
     // 20^3 7.0 -> 6.5 ms; cells of edge 6 to 30 mixed, the largest in HBM either way, 56.5 -> 82.3 ms.
     // hea_batch_autotune compares the alternatives on the batch at hand.
-    if (rc == HEA_OK) rc = batch_configure(b, 0, HEA_BATCH_MIN_BLOCKS);
-    if (rc == HEA_OK && std::any_of(b->h_structs.begin(), b->h_structs.end(), [](const BatchStruct &d) { return d.hbm; }))
-        rc = batch_configure(b, 1, HEA_BATCH_MIN_BLOCKS);
+    size_t budget = 0;
+    if (rc == HEA_OK) rc = batch_smem_budget(&budget);
+    if (rc == HEA_OK) {
+        const bool staged = std::all_of(b->h_structs.begin(), b->h_structs.end(), [&](const BatchStruct &d) {
+            return batch_job_smem(d.c.occ_stride, d.T, d.c.num_shells, b->block / 32, false) <= budget;
+        });
+        rc = batch_configure(b, staged ? 0 : 1, HEA_BATCH_MIN_BLOCKS);
+    }
     if (rc != HEA_OK) {
         delete b;
         return rc;

@@ -2300,11 +2300,11 @@ int hea_batch_create(const hea_problem *problems, const hea_params *params, int3
     }
     if (rc == HEA_OK) {
         rc = batch_populations(b, ahead);
-        if (rc == HEA_ERR_NOMEM && ahead > 1) {
+        while (rc == HEA_ERR_NOMEM && ahead > 1) {
             cudaGetLastError();
             for (void *p : b->buffers) dev_free(p);
             b->buffers.clear();
-            rc = batch_populations(b, 1);
+            rc = batch_populations(b, --ahead);
         }
     }
     for (const BatchStruct &d : b->h_structs) hist_total += hist_bytes_of(d.c, 2 * d.P);

@@ -1,0 +1,65 @@
+"""Device memory of the populations searched ahead: what a batch takes where the
+device has little, and what many plans take together."""
+import gc
+
+import numpy as np
+import pytest
+import torch
+
+import pyhea_b200 as hb
+from pyhea_b200 import lattice as L
+from pyhea_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+MIB = 1 << 20
+GIB = 1 << 30
+
+
+def free_bytes():
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def give_back():
+    gc.collect()
+    hb.lib.hea_release_cached_memory()
+    torch.cuda.empty_cache()
+
+
+def structure(lattice, cell, types, seed=0):
+    rng = np.random.default_rng(seed)
+    species = W.dirichlet_counts(rng, types, L.num_sites(lattice, cell))
+    target = W.projected_target(rng, species / species.sum(), 0.1)
+    return hb.Problem.from_lattice(lattice, cell, species, W.WEIGHTS, target)
+
+
+def test_a_batch_short_of_memory_takes_what_fits():
+    """Four populations ahead do not fit and two do: the batch takes more than the one it needs, and
+    searches the same."""
+    pb = structure(L.BCC, 30, 4)  # 54 000 sites: 486 KB a slot
+    P = 256
+    slot = P * 9 * pb.num_sites  # one population's histograms and occupancies
+    prm = [dict(num_solutions=P, total_iter=4, parallel_task=64, converge_depth=1, max_rounds=2)]
+
+    def taken():
+        give_back()
+        before = free_bytes()
+        b = hb.Batch([pb], prm)
+        used = before - free_bytes()
+        b.run([5])
+        got = b.read(0)
+        b.close()
+        return used, got
+
+    full, want = taken()
+    assert full > 4.9 * slot  # survivors and four populations
+    give_back()
+    spare = int(3.6 * slot)
+    block = torch.empty(free_bytes() - spare, dtype=torch.uint8, device="cuda")
+    short, got = taken()
+    del block
+    give_back()
+    assert 2.9 * slot < short < 3.6 * slot
+    np.testing.assert_array_equal(got[0], want[0])
+    np.testing.assert_array_equal(got[1], want[1])

@@ -149,6 +149,55 @@ void dev_free(void *p)
 }
 
 // ---------------------------------------------------------------------------
+// Populations searched ahead beyond the first of each search take memory that
+// it could do without.  All live plans and batches of a device together take at
+// most kAheadTotalBytes of it; one that is made when it is used up searches
+// fewer ahead (the same results, slower), and finds the rest of the device as if
+// nobody searched ahead.
+// ---------------------------------------------------------------------------
+constexpr size_t kAheadTotalBytes = (size_t)16 << 30;
+class AheadShare {
+public:
+    ~AheadShare() { give(); }
+    // `bytes` of the current device's total, instead of what it holds; false when there is not as much left.
+    bool take(size_t bytes)
+    {
+        give();
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess) return false;
+        Total &t = total();
+        std::lock_guard<std::mutex> lk(t.mu);
+        size_t &held = t.held[dev];
+        if (bytes > kAheadTotalBytes - held) return false;
+        held += bytes;
+        dev_ = dev;
+        bytes_ = bytes;
+        return true;
+    }
+    void give()
+    {
+        if (!bytes_) return;
+        Total &t = total();
+        std::lock_guard<std::mutex> lk(t.mu);
+        t.held[dev_] -= bytes_;
+        bytes_ = 0;
+    }
+
+private:
+    struct Total {
+        std::mutex mu;
+        std::map<int, size_t> held;
+    };
+    static Total &total()
+    {
+        static Total *t = new Total;  // never destroyed, like the block cache
+        return *t;
+    }
+    int dev_ = 0;
+    size_t bytes_ = 0;
+};
+
+// ---------------------------------------------------------------------------
 // Streams (each with two events) of finished plans, kept for the next plan in
 // the same context: a call that makes a plan of its own otherwise spends more
 // on creating and destroying them than on a small structure's kernels
@@ -1037,6 +1086,7 @@ struct hea_plan {
     // slots may be rewritten, its search has ended
     enum { kFree, kDone };
     std::vector<Queue> ahead;
+    AheadShare ahead_memory;
     uint8_t *occ = nullptr, *out_occ = nullptr;
     int32_t *cnt = nullptr, *order = nullptr, *scratch = nullptr;
     double *f2 = nullptr, *out_f2 = nullptr;
@@ -1443,7 +1493,8 @@ int plan_autotune(hea_plan *pl, bool measure)
 // leaves the chip waiting for each iteration's slowest searches, merge and
 // survivors, and a population smaller than the chip never fills it; enough of
 // them keep two chips' worth of CTAs queued.  Bounded by the iterations, by
-// kMaxAhead streams and by kAheadBytes of population buffers beyond the first.
+// kMaxAhead streams and by kAheadBytes of population buffers beyond the first
+// (AheadShare: of all plans and batches together).
 // Measured on B200, one population in flight -> this rule, whole call or run:
 // FCC 10^3 (128 solutions x 256 tasks, 10 iterations) 9.64 -> 3.77 ms, a
 // 5148-site box (48 x 200, 6 iterations) 5.23 -> 2.17 ms, BCC 20^3 (256 x 512,
@@ -1451,7 +1502,13 @@ int plan_autotune(hea_plan *pl, bool measure)
 constexpr int kMaxAhead = 16;
 constexpr size_t kAheadBytes = (size_t)4 << 30;
 
-int plan_lookahead(const hea_plan *pl, int *out)
+// Bytes of one of a plan's populations (site histograms and occupancies).
+size_t plan_population_bytes(const hea_plan *pl)
+{
+    return (hist_bytes_of(pl->dt.c, 1) + pl->dt.c.occ_stride) * (size_t)pl->P;
+}
+
+int plan_lookahead(hea_plan *pl, int *out)
 {
     const DeviceTables &dt = pl->dt;
     const hea_params &prm = pl->prm;
@@ -1467,9 +1524,10 @@ int plan_lookahead(const hea_plan *pl, int *out)
             &per_sm, dt.mc, pl->mc_block, mc_smem(dt.c.occ_stride, dt.T, dt.S, pl->mc_block / 32)));
     }
     const int64_t want = (2 * (int64_t)sms * std::max(1, per_sm) + pl->P - 1) / pl->P;
-    const size_t each = (hist_bytes_of(dt.c, 1) + dt.c.occ_stride) * (size_t)pl->P;
+    const size_t each = plan_population_bytes(pl);
     const int64_t room = 1 + (int64_t)(kAheadBytes / each);
     *out = (int)std::max<int64_t>(1, std::min<int64_t>({std::max<int64_t>(2, want), room, kMaxAhead, prm.total_iter}));
+    while (*out > 1 && !pl->ahead_memory.take(each * (size_t)(*out - 1))) --*out;
     return HEA_OK;
 }
 
@@ -1493,6 +1551,7 @@ int plan_create(const hea_problem *pb, const hea_params *prm, int slots, hea_pla
             ahead = (ahead + 1) / 2;
             cudaGetLastError();
             pl->free_buffers();
+            pl->ahead_memory.take(plan_population_bytes(pl) * (size_t)(ahead - 1));
             rc = plan_alloc(pl, pl->P * (ahead + 1));
         }
         if (rc == HEA_OK) rc = plan_streams(pl, ahead);
@@ -2076,6 +2135,7 @@ struct hea_batch {
     std::vector<DeviceTables *> tables;
     std::vector<BatchStruct> h_structs;
     std::vector<void *> buffers;  // every device allocation of the batch
+    AheadShare ahead_memory;
     BatchStruct *d_structs = nullptr;
     BatchState *d_states = nullptr;
     BatchJob *d_jobs = nullptr;
@@ -2289,22 +2349,27 @@ int hea_batch_create(const hea_problem *problems, const hea_params *params, int3
         b->h_structs.push_back(d);
         b->total_jobs += (unsigned long long)P * (2 * d.I + 1);
     }
-    // new populations in flight: as many as kBatchAheadBytes of populations allow, or fewer where the
-    // device has no room for them
-    int ahead = kBatchAhead;
-    for (; rc == HEA_OK && ahead > 1; --ahead) {
+    // new populations in flight: as many as kBatchAheadBytes of populations allow (and AheadShare, of
+    // those beyond the first), or fewer where the device has no room for them
+    const auto populations = [b](int n) {  // bytes of the survivors and n populations of every structure
         size_t bytes = 0;
         for (const BatchStruct &d : b->h_structs)
-            bytes += (hist_bytes_of(d.c, 1) + 2 * (size_t)d.c.num_sites) * d.P * (std::max(1, std::min(ahead, d.I)) + 1);
-        if (bytes <= kBatchAheadBytes) break;
-    }
+            bytes += (hist_bytes_of(d.c, 1) + 2 * (size_t)d.c.num_sites) * d.P * (std::max(1, std::min(n, d.I)) + 1);
+        return bytes;
+    };
+    int ahead = rc == HEA_OK ? kBatchAhead : 1;
+    while (ahead > 1 && (populations(ahead) > kBatchAheadBytes ||
+                         !b->ahead_memory.take(populations(ahead) - populations(1))))
+        --ahead;
     if (rc == HEA_OK) {
         rc = batch_populations(b, ahead);
         while (rc == HEA_ERR_NOMEM && ahead > 1) {
             cudaGetLastError();
             for (void *p : b->buffers) dev_free(p);
             b->buffers.clear();
-            rc = batch_populations(b, --ahead);
+            --ahead;
+            b->ahead_memory.take(populations(ahead) - populations(1));
+            rc = batch_populations(b, ahead);
         }
     }
     for (const BatchStruct &d : b->h_structs) hist_total += hist_bytes_of(d.c, 2 * d.P);

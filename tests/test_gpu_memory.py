@@ -63,3 +63,32 @@ def test_a_batch_short_of_memory_takes_what_fits():
     assert 2.9 * slot < short < 3.6 * slot
     np.testing.assert_array_equal(got[0], want[0])
     np.testing.assert_array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("form", ["plan", "batch"])
+def test_many_searches_leave_the_device_its_memory(form):
+    """Each alone would search several populations ahead; all together take 16 GiB for those beyond the
+    first, and what they return comes back when they close."""
+    if form == "plan":
+        pb = structure(L.FCC, 80, 3)  # 2 048 000 sites
+        count, P = 12, 8
+        make = lambda: hb.Plan(pb, P, 16, 64, 2, max_rounds=2)
+    else:
+        pb = structure(L.FCC, 80, 3)
+        count, P = 8, 64
+        make = lambda: hb.Batch([pb], [dict(num_solutions=P, total_iter=16, parallel_task=64, converge_depth=1)])
+    each = 9 * P * pb.num_sites
+    for _ in range(2):
+        give_back()
+        before = free_bytes()
+        kept, used = [], []
+        for _ in range(count):
+            kept.append(make())
+            used.append(before - free_bytes())
+        extra = used[-1] - count * 2.2 * each  # beside survivors, one population and the reading buffer
+        assert extra < 16 * GIB
+        assert used[0] > 3 * each  # the first ones search ahead
+        for k in kept:
+            k.close()
+    give_back()
+    assert before - free_bytes() < 64 * MIB

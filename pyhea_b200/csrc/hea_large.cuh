@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(512, 2) mc_large_kernel(const __grid_constant_
     while (miss < g.depth && round < g.max_rounds) {
         Record *rr = rec + (round & 1) * nwarps;
         Record &mine = rr[warp];
-        if (lane == 0) mine.lo = mine.hi = kNoSwap;
+        if (lane == 0) mine.lo = mine.hi = kEmpty;
         __syncwarp();
         const int32_t *cold = cnt2 + buf * NCP;
         for (int q0 = qlo + warp * 32; q0 < qhi; q0 += blockDim.x) {

@@ -438,6 +438,9 @@ __device__ __forceinline__ double fitness_of_counts(const SearchConst &c, const 
 // checks (SearchConst::screen_floor).
 // ---------------------------------------------------------------------------
 constexpr float kNoSwap = 3.0e38f;  // lo and hi of no proposal, or of one that does not improve
+// lo and hi of a warp's record before a pass has found a proposal for it: above every proposal's hi, also where
+// all are exact (screen_floor) and hi is 3e38, so that an empty record is never compared with (keep_best)
+constexpr float kEmpty = __builtin_huge_valf();
 constexpr float kScreenEps = 32.0f / 16777216.0f;
 
 // Layout of the FP32 table, in floats: rows of (k, a, b), within a row species
@@ -1386,9 +1389,7 @@ __device__ __forceinline__ void keep_best(const SearchConst &c, const int32_t *c
         int win = __ffs(cand) - 1;
         if (cand & (cand - 1)) win = resolve<T, L>(c, cnt, (cand >> lane) & 1u, least < 0.0f, r.task, r.ab, r.p, r.q);
         if (lane == win) {
-            // an empty record (lo = kNoSwap: no pass before found a D < 0) has no proposal to compare with, and
-            // where every proposal is exact (screen_floor) its hi equals theirs
-            bool take = !more || mine.lo == kNoSwap || r.hi < mine.lo;
+            bool take = !more || r.hi < mine.lo;  // mine.lo = kEmpty: no pass before found a D < 0
             if (!take && r.lo <= mine.hi) {  // an earlier pass's best too near to tell; on equal D it has the lower task
                 double before = 0.0, D = 0.0;
 #pragma unroll 1
@@ -1496,7 +1497,7 @@ __device__ __forceinline__ McTally mc_rounds(const SearchConst &c, const int4 *_
     while (miss < depth && round < max_rounds && !(kYield && cur <= rs.tol2)) {
         Record *rr = rec + (round & 1) * nwarps;
         Record &mine = rr[warp];  // this warp's best proposal of the round
-        if (lane == 0) mine.lo = mine.hi = kNoSwap;
+        if (lane == 0) mine.lo = mine.hi = kEmpty;
         __syncwarp();
         const int32_t *cold = cnt2 + buf * NCP;
         // passes of blockDim tasks; lane q of a pass scores task q (warp-uniform trip count)

@@ -862,14 +862,20 @@ size_t hist_bytes_of(const SearchConst &c, int64_t slots)
     return (size_t)slots * c.num_sites * hist_words(c.num_types, c.num_shells, c.lat.L > 0) * sizeof(uint64_t);
 }
 
-// Whether a structure streams its histogram loads (SearchConst::hist_stream).
-// `total_bytes` is the histogram memory of every structure resident with it
-// (its own alone for a plan).  Until that total passes twice the L2 size the
-// structures keep their lines cached; beyond it, those with more than
-// kSharedStreamBytes of their own stream, so that the lines of the smaller
-// ones stay.  Measured on batches of 8 FCC 30^3 structures (108 000
-// sites, 442 MB of histograms): 81.8 -> 74.2 ms (4 species), 94.6 -> 85.5 ms (6);
-// FCC 100^3 36.4 -> 35.0 ms.
+// Whether a structure of a batch or a server streams its histogram loads
+// (SearchConst::hist_stream).  Bytes are those of a structure's survivors and one
+// new population (those queued further ahead mostly wait); `total_bytes` is the
+// sum over all structures that run with it.  Until that passes twice the L2 size
+// they keep their lines cached; beyond it, those with more than
+// kSharedStreamBytes of their own stream, so that the lines of the smaller ones
+// stay.  Measured, cached -> this rule (total MB): 8 FCC 30^3 (843) 56.7 -> 50.3 ms,
+// 40 cells of edge 6 to 30 (1055) 58.4 -> 57.3; all streaming: 8 FCC 20^3 (250) 10.9
+// -> 11.5, the 40 cells 58.9, 24 cells of edge 12 to 20 (320) 16.2 -> 16.5; a line at
+// 16 MiB 58.8 and at 256 MiB 57.7 on the 40 cells.
+// Plans never stream: one structure's searches read their own lines again.
+// Streamed -> cached: FCC 30^3, 64 solutions x 8 iterations 34.3 -> 28.9 ms, 592 x 1
+// 38.4 -> 33.3, FCC 60^3 (cluster search) 16 x 4 20.5 -> 17.3, FCC 100^3 32 x 1 35.4 ->
+// 35.5, fourteen others between level and 18 % in favour of cached.
 constexpr size_t kSharedStreamBytes = (size_t)64 << 20;
 
 uint32_t stream_histograms(size_t hist_bytes, size_t total_bytes)
@@ -1556,8 +1562,6 @@ int plan_create(const hea_problem *pb, const hea_params *prm, int slots, hea_pla
         }
         if (rc == HEA_OK) rc = plan_streams(pl, ahead);
         if (slots == 0) slots = pl->P * (ahead + 1);
-        const size_t hist_bytes = hist_bytes_of(pl->dt.c, slots);
-        pl->dt.c.hist_stream = stream_histograms(hist_bytes, hist_bytes);
         if (rc == HEA_OK) rc = plan_clear(pl, slots);
     }
     if (rc == HEA_OK) rc = plan_autotune(pl, (prm->flags & HEA_FLAG_AUTOTUNE) != 0);
@@ -2316,7 +2320,7 @@ int hea_batch_create(const hea_problem *problems, const hea_params *params, int3
     hea_batch *b = new (std::nothrow) hea_batch();
     if (!b) return fail(HEA_ERR_NOMEM, "out of host memory");
     b->count = count;
-    size_t hist_total = 0;  // site-histogram bytes of all structures (stream_histograms)
+    size_t hist_total = 0;  // stream_histograms' total
     int rc = HEA_OK;
     for (int i = 0; i < count && rc == HEA_OK; ++i) {
         rc = validate_params(&params[i]);
@@ -2619,7 +2623,7 @@ struct ServerRequest {
     int lattice = -1, cell = 0, shell_set = 0;
     int slot = -1, hbm = 0;
     size_t off = 0, bytes = 0;
-    size_t hist_bytes = 0;  // site-histogram bytes of the placed request
+    size_t hist_bytes = 0;  // stream_histograms' bytes of the placed request
     unsigned long long ring_load = 0;  // ring slots it holds at its level
     double t_submit = 0, t_admit = 0, t_finish = 0, device_ms = 0;
     int iterations = 0;
@@ -2698,7 +2702,7 @@ struct hea_server {
     std::vector<void *> buffers;
     uint8_t *arena = nullptr;
     ArenaHeap heap;
-    size_t hist_placed = 0;  // site-histogram bytes of the placed requests (stream_histograms)
+    size_t hist_placed = 0;  // stream_histograms' total of the placed requests
     BatchStruct *d_structs = nullptr;
     BatchState *d_states = nullptr;
     BatchJob *d_jobs = nullptr;

@@ -662,9 +662,10 @@ __device__ __forceinline__ uint64_t hist_species_bits(int a)
     return ((uint64_t)(a & 3) << 62) | ((uint64_t)(a >> 2) << 31);
 }
 
-// Two sites' entries, through L2.  Structures whose histograms are far larger
-// than L2 (SearchConst::hist_stream, set by the host) read them evict-first, so
-// that random lines from DRAM do not push out those that are read again.
+// Two sites' entries, through L2.  In batches whose histograms are far larger
+// than L2 the large structures (SearchConst::hist_stream, set by the host) read
+// them evict-first, so that random lines from DRAM do not push out those that are
+// read again.
 template <int W>
 __device__ __forceinline__ void load_hist_pair(const SearchConst &c, const uint64_t *hist, uint32_t s1, uint32_t s2,
                                                HistEntry<W> &p, HistEntry<W> &q)

@@ -775,11 +775,14 @@ cudaError_t allow_max_smem(F *func)
 // Constants of the FP32 screening (score_delta): its scale, and whether its
 // bound holds -- every Q and Cq at most about 1 and far above FP32's smallest
 // normal number, or zero, and no target so large that an L leaves its range.
-// (With |E| <= 1e6 an L stays below (|E| + N) / R_max < 1e20.)
+// (With |E| <= 1e6 an L stays below (|E| + N) / R_max < 1e20.)  And targets that
+// differ across the diagonal do so by no more than the bound covers (the last
+// paragraph above score_delta): |E_ij - E_ji| + 2 C R <= 2^30 R, C <= Z min(n_i, n_j).
 void fill_screen_const(const hea_problem *pb, SearchConst &c)
 {
     const int T = pb->num_types, S = pb->num_shells;
     double qmax = 0.0, qmin = HUGE_VAL, emax = 0.0;
+    bool covered = true;
     for (int k = 0; k < S; ++k)
         for (int e = 0; e < T * T; ++e) {
             const double q = 2.0 * c.w[k] * c.R[k * T * T + e] * c.R[k * T * T + e];
@@ -789,13 +792,16 @@ void fill_screen_const(const hea_problem *pb, SearchConst &c)
             }
             if (c.w[k] > 0.0) qmin = std::min(qmin, q);  // an underflow to 0
             emax = std::max(emax, std::fabs(c.E[k * T * T + e]));
+            const int i = e / T, j = e % T;
+            const double apart = std::fabs(c.E[(k * T + i) * T + j] - c.E[(k * T + j) * T + i]);
+            const double most = (double)pb->shell_sizes[k] * std::min(pb->species[i], pb->species[j]);
+            if (apart > 0.0 && apart + 2.0 * most * c.R[k * T * T + e] > std::ldexp(c.R[k * T * T + e], 30)) covered = false;
         }
     int exponent = 0;
     if (qmax > 0.0 && std::isfinite(qmax)) std::frexp(qmax, &exponent);
     c.screen_scale = std::ldexp(1.0, -exponent);
     const bool fits = std::isfinite(qmax) && std::isfinite(c.screen_scale) && c.screen_scale > 0.0 && emax <= 1e6 &&
-                       (qmax == 0.0 || qmin * c.screen_scale >= std::ldexp(1.0, -100))
-;
+                      covered && (qmax == 0.0 || qmin * c.screen_scale >= std::ldexp(1.0, -100));
     c.screen_floor = fits ? 0.0f : kNoSwap;
     if (!fits) c.screen_scale = 0.0;
     for (int k = 0; k < S; ++k)

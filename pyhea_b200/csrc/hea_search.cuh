@@ -436,6 +436,14 @@ __device__ __forceinline__ double fitness_of_counts(const SearchConst &c, const 
 // kept with the table; 32 leaves room for the roundings of e itself and of D.
 // It holds while the table's values stay in FP32's range, which the host
 // checks (SearchConst::screen_floor).
+//
+// D itself is rounded too.  Where E is symmetric, d_it + d_ti = 2 d_it, rounded
+// as the table's one fma rounds it: relative steps of 2^-53, far inside what 32
+// leaves over 24.  Else the two differ by up to 2^-52 (|E_it - E_ti| / 2 + C R)
+// however small the sum is: by eta R_it, say, which moves D by at most 3 eta B
+// (|u| >= 1; the cross terms by Cq and the larger of Q_a, Q_b, since R_aa R_bb =
+// R_ab^2).  8 delta B is left for it, so eta <= 2^-23 is covered, which the host
+// checks as well; beyond it every D is exact.
 // ---------------------------------------------------------------------------
 constexpr float kNoSwap = 3.0e38f;  // lo and hi of no proposal, or of one that does not improve
 // lo and hi of a warp's record before a pass has found a proposal for it: above every proposal's hi, also where

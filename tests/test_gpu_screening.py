@@ -5,6 +5,8 @@ weights or targets outside FP32's range, six species in three shells (both
 histogram widths) -- and where a round takes several passes (CTAs smaller than
 the round, on one CTA and on a cluster, in both draw modes), with and without
 the screening."""
+from fractions import Fraction
+
 import numpy as np
 import pytest
 
@@ -110,3 +112,61 @@ def test_batch_passes_with_every_proposal_exact(species, shells, weight, scale):
             np.testing.assert_array_equal(occ, wocc)
             np.testing.assert_array_equal(fit, np.sqrt(wf2))
     b.close()
+
+
+def fma(a, b, c):
+    return float(Fraction(a) * Fraction(b) + Fraction(c))
+
+
+def asymmetric_target(op, C, rng, x):
+    """Two species, one shell: targets with 1 - target = C R +- x off the diagonal (about), such that the swap
+    with u = (1, -1) has D < 0 by the rounding of d_01 + d_10 alone (about 2^-53 x), while the sums rounded once
+    put D above zero by more than the screening's bound."""
+    R = op.R[0]
+    r = R[0, 1]
+    quad = 4 * R[0, 0] ** 2 + 4 * R[1, 1] ** 2 + 8 * r ** 2
+    bound = 2.0 ** -19 * quad * 3.1  # z: the sums s_it are about 2 R
+    for _ in range(10000):
+        off = x * rng.uniform(0.5, 1.0)
+        E = np.array([[C[0, 0] * r + r, C[0, 1] * r - r + off], [C[1, 0] * r - r - off, C[1, 1] * r + r]])
+        E = 1.0 - (1.0 - E)
+        s = lambda i, j: Fraction(E[i, j]) + Fraction(E[j, i]) - 2 * int(C[i, j]) * Fraction(r)  # noqa: E731
+        # D = -2 r (s_00 + s_11 - 2 s_01) + quad = 1.6 bounds
+        E[0, 0] = (float(2 * s(0, 1) - s(1, 1)) + (quad - 1.6 * bound) / (2 * r)) / 2 + C[0, 0] * r
+        E = 1.0 - (1.0 - E)
+        d = lambda i, j: fma(-float(C[i, j]), r, E[i, j])  # noqa: E731
+        G = lambda i, t: r * (d(i, t) + d(t, i))  # noqa: E731
+        D = 0.0
+        for t, u in ((0, 1.0), (1, -1.0)):
+            D = fma(u, fma(u, 4.0 * (r * r), -2.0 * (G(0, t) - G(1, t))), D)
+        D = fma(4.0, 2.0 * (r * r), D)
+        once = lambda i, j: fma(-float(C[i, j]), 2 * r, E[i, j] + E[j, i])  # noqa: E731
+        if D < 0.0 and -2.0 * r * (once(0, 0) + once(1, 1) - 2.0 * once(0, 1)) + quad > 1.4 * bound:
+            return 1.0 - E
+    raise AssertionError("no such target")
+
+
+@pytest.mark.parametrize("cell,x", [(10, 9e5), (20, 1e2), (50, 1e2), (50, 9e5)])
+def test_asymmetric_targets(cell, x):
+    """Targets far apart across the diagonal, from a state that meets their mean: the bound does not cover
+    the rounding of d_01 + d_10 where they are too far apart, and every proposal is then exact."""
+    species = [2 * cell ** 3] * 2
+    nbor, sizes = L.neighbors(L.FCC, cell, L.SHELLS_REFERENCE)
+    row = int(sizes[0])
+    oracle = lambda target: ho.Problem(nbor[:, :row], sizes[:1], species, [1.0], target.reshape(1, 4))  # noqa: E731
+    op = oracle(np.zeros((2, 2)))
+    occ = op.generate(5, 0, 0)
+    C = op.recount(occ)[0]
+    if x < 1e3 or cell == 10:  # covered
+        r = op.R[0, 0, 1]
+        target = 1.0 - (C * r + np.array([[r, x - r], [-x - r, r]]))
+    else:
+        target = asymmetric_target(op, C, np.random.default_rng(cell), x)
+    op = oracle(target)
+    want = op.mc(9, 2 << 16, occ, 300, 2, max_rounds=4, trace_cap=4)
+    gp = hb.Problem(nbor, sizes, species, [1.0], target.reshape(1, 4))
+    for p in (gp, hb.Problem(nbor, sizes, species, [1.0], target.reshape(1, 4), recognize=False)):
+        got = hb.local_search(p, 9, 2, occ[None], 300, 2, max_rounds=4, trace_cap=4)
+        assert [t[:4] for t in got["trace"][0]] == [t[:4] for t in want["trace"]]
+        np.testing.assert_array_equal(got["occ"][0], want["occ"])
+        assert got["f2"][0] == want["f2"]

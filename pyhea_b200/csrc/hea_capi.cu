@@ -878,10 +878,6 @@ size_t hist_bytes_of(const SearchConst &c, int64_t slots)
 // 40 cells of edge 6 to 30 (1055) 58.4 -> 57.3; all streaming: 8 FCC 20^3 (250) 10.9
 // -> 11.5, the 40 cells 58.9, 24 cells of edge 12 to 20 (320) 16.2 -> 16.5; a line at
 // 16 MiB 58.8 and at 256 MiB 57.7 on the 40 cells.
-// Plans never stream: one structure's searches read their own lines again.
-// Streamed -> cached: FCC 30^3, 64 solutions x 8 iterations 34.3 -> 28.9 ms, 592 x 1
-// 38.4 -> 33.3, FCC 60^3 (cluster search) 16 x 4 20.5 -> 17.3, FCC 100^3 32 x 1 35.4 ->
-// 35.5, fourteen others between level and 18 % in favour of cached.
 constexpr size_t kSharedStreamBytes = (size_t)64 << 20;
 
 uint32_t stream_histograms(size_t hist_bytes, size_t total_bytes)
@@ -1514,6 +1510,44 @@ int plan_autotune(hea_plan *pl, bool measure)
 constexpr int kMaxAhead = 16;
 constexpr size_t kAheadBytes = (size_t)4 << 30;
 
+// Searches of a plan that are resident at once: CTAs, or clusters of two 512-thread CTAs per SM.
+int plan_resident(const hea_plan *pl, int64_t *out)
+{
+    const DeviceTables &dt = pl->dt;
+    int dev = 0, sms = 0, per_sm = 1;
+    HEA_CUDA(cudaGetDevice(&dev));
+    HEA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (dt.large) {
+        *out = 2 * sms / cluster_size(pl->prm.parallel_task);
+    } else {
+        HEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &per_sm, dt.mc, pl->mc_block, mc_smem(dt.c.occ_stride, dt.T, dt.S, pl->mc_block / 32)));
+        *out = (int64_t)sms * std::max(1, per_sm);
+    }
+    return HEA_OK;
+}
+
+// Whether a plan of `slots` rows streams its histogram loads: when the searches
+// that are resident at once hold more than six times the L2, which only the
+// cluster path reaches.  Rows that wait do not count.  Cached against streamed,
+// whole searches of 4 species: 37 searches of FCC 100^3 (1.18 GB) 2268 against 2247
+// ms (32 solutions x 3 iterations), 3025 against 2986 (64 x 2); of FCC 80^3 (606 MB)
+// level (1106 against 1104, 1475 against 1478); below, cached: FCC 60^3 (256 MB) 577
+// against 588 and 310 against 306, capped searches of it 17.3 against 20.5, FCC
+// 30^3 on the shared-memory path (256 MB) 43.4 against 51.3, 28.9 against 34.3.
+int plan_streams_histograms(const hea_plan *pl, int slots, uint32_t *out)
+{
+    *out = 0;
+    if (!pl->dt.large) return HEA_OK;
+    int dev = 0, l2 = 0;
+    int64_t resident = 0;
+    HEA_CUDA(cudaGetDevice(&dev));
+    HEA_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
+    HEA_TRY(plan_resident(pl, &resident));
+    *out = hist_bytes_of(pl->dt.c, std::min<int64_t>(slots, resident)) > 6 * (size_t)l2 ? 1u : 0u;
+    return HEA_OK;
+}
+
 // Bytes of one of a plan's populations (site histograms and occupancies).
 size_t plan_population_bytes(const hea_plan *pl)
 {
@@ -1522,20 +1556,12 @@ size_t plan_population_bytes(const hea_plan *pl)
 
 int plan_lookahead(hea_plan *pl, int *out)
 {
-    const DeviceTables &dt = pl->dt;
     const hea_params &prm = pl->prm;
     *out = 1;
     if (prm.total_iter < 2) return HEA_OK;
-    int dev = 0, sms = 0, per_sm = 1;
-    HEA_CUDA(cudaGetDevice(&dev));
-    HEA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (dt.large) {  // two 512-thread CTAs per SM, a cluster of up to 8 per solution
-        sms = 2 * sms / cluster_size(prm.parallel_task);
-    } else {
-        HEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, dt.mc, pl->mc_block, mc_smem(dt.c.occ_stride, dt.T, dt.S, pl->mc_block / 32)));
-    }
-    const int64_t want = (2 * (int64_t)sms * std::max(1, per_sm) + pl->P - 1) / pl->P;
+    int64_t resident = 0;
+    HEA_TRY(plan_resident(pl, &resident));
+    const int64_t want = (2 * resident + pl->P - 1) / pl->P;
     const size_t each = plan_population_bytes(pl);
     const int64_t room = 1 + (int64_t)(kAheadBytes / each);
     *out = (int)std::max<int64_t>(1, std::min<int64_t>({std::max<int64_t>(2, want), room, kMaxAhead, prm.total_iter}));
@@ -1568,6 +1594,7 @@ int plan_create(const hea_problem *pb, const hea_params *prm, int slots, hea_pla
         }
         if (rc == HEA_OK) rc = plan_streams(pl, ahead);
         if (slots == 0) slots = pl->P * (ahead + 1);
+        if (rc == HEA_OK) rc = plan_streams_histograms(pl, slots, &pl->dt.c.hist_stream);
         if (rc == HEA_OK) rc = plan_clear(pl, slots);
     }
     if (rc == HEA_OK) rc = plan_autotune(pl, (prm->flags & HEA_FLAG_AUTOTUNE) != 0);

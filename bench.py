@@ -76,21 +76,22 @@ HBM_FALLBACK_GBS = 6650.0
 #   inst   smsp__inst_executed.sum (warp instructions)        -> roofline.issue_frac
 #   dram_read  dram__bytes_read.sum                           -> roofline.dram_random (batched)
 # mc_kernel<5, ImplicitShells<3>> (the plain structure's table is recognised as a BCC lattice's): the
-# first local-search launch of `python bench.py --case plain --iters 1` (203.72 M evaluations):
-# 37.02 MB + 4.27 MB DRAM, 418.07 M L2 sectors, 3.6224 G warp instructions.  batch_kernel: the launch
+# first local-search launch of `python bench.py --case plain --iters 8` (203.72 M evaluations, 256
+# threads per CTA as in the bench's run): 37.34 MB + 3.94 MB DRAM, 418.08 M L2 sectors, 3.1827 G warp
+# instructions.  batch_kernel: the launch
 # of `python bench.py --case batch --count 64 --iters 10`, the bench's batch configuration (6268.46 M
 # evaluations, lattice tables recognised): 842.36 GB + 57.09 GB DRAM, 56.92 G L2 sectors, 166.75 G
 # warp instructions.  dram_random_probe_kernel (hea_dram_random_probe over 4 GiB, 77.59 M
-# random 16-byte loads): 9.833 GB DRAM read, i.e. 126.7 B per load (each load fetches a 128-byte line).
+# random 8-byte loads): 9.724 GB DRAM read, i.e. 125.3 B per load (each load fetches a 128-byte line).
 KERNEL_COUNTERS = {
-    "plain_gpu": {"dram": (37.02e6 + 4.27e6) / 203.72e6, "l2": 418.07e6 * 32.0 / 203.72e6,
-                  "inst": 3.6224e9 / 203.72e6,
-                  "capture": "mc_kernel, first local-search launch of bench.py --case plain --iters 1"},
+    "plain_gpu": {"dram": (37.34e6 + 3.94e6) / 203.72e6, "l2": 418.08e6 * 32.0 / 203.72e6,
+                  "inst": 3.1827e9 / 203.72e6,
+                  "capture": "mc_kernel, first local-search launch of bench.py --case plain --iters 8"},
     "batched": {"dram": (842.36e9 + 57.09e9) / 6268.46e6, "l2": 56.92e9 * 32.0 / 6268.46e6,
                 "inst": 166.75e9 / 6268.46e6, "dram_read": 842.36e9 / 6268.46e6,
                 "capture": "batch_kernel, bench.py --case batch --count 64 --iters 10"},
 }
-DRAM_BYTES_PER_RANDOM_LOAD = 9.833e9 / 77.594624e6
+DRAM_BYTES_PER_RANDOM_LOAD = 9.7245e9 / 77.594624e6
 L2_PROBE_BYTES = 32 << 20  # fits in L2 (126 MB) with room to spare
 
 
@@ -446,7 +447,7 @@ def measure_batched(steps, warmup, l2_peak=None, implicit=False, select=None):
     roof = roofline_of("batch_kernel (persistent job engine)", KERNEL_COUNTERS["batched"], b_ev, b_ms / 1000.0,
                        bpe, steps, clocks, l2_peak, sm_count())
     # the regime that binds the batch: most of its evaluations are on structures whose site
-    # histograms stay in DRAM, read at random; random 16-byte DRAM loads are measured here by the
+    # histograms stay in DRAM, read at random; random 8-byte DRAM loads are measured here by the
     # library's probe and converted to DRAM bytes with the probe's captured bytes per load (the
     # batch's own DRAM traffic also holds streaming reads, so its fraction can exceed 1)
     loads_per_s = hb.dram_random_probe(4 << 30, 256)

@@ -163,11 +163,6 @@ struct JobEnd {
     int32_t yielded, round, miss;
 };
 
-// One job of a structure with species count T and layout L.  Shared memory:
-// [occ (occ_stride + 16), unless hbm] | search_smem_tail(T, S, nwarps) (delta
-// table, swap records, two count buffers).
-// The rounds of a job's local search in a call of their own: values the job
-// needs only before and after the search stay out of the loop's registers.
 // One recount instance for the layouts that share it.
 template <int T, int S, RecountForm kNeighbors>
 __device__ __noinline__ void batch_recount(const SearchConst &c, const int4 *nbor, const uint8_t *occ, int32_t *cnt,
@@ -176,6 +171,8 @@ __device__ __noinline__ void batch_recount(const SearchConst &c, const int4 *nbo
     block_recount<T, S, kNeighbors>(c, nbor, occ, cnt, hist);
 }
 
+// The rounds of a job's local search in a call of their own: values the job
+// needs only before and after the search stay out of the loop's registers.
 template <int T, class L>
 __device__ __noinline__ McTally batch_search(const SearchConst &c, const BatchStruct &d, uint8_t *occ, int32_t *cnt2,
                                              const DeltaTab<T, L::S> tab, void *rec, uint32_t stream, double cur,
@@ -185,6 +182,9 @@ __device__ __noinline__ McTally batch_search(const SearchConst &c, const BatchSt
                                  McTrace{nullptr, nullptr, 0}, rs, hist, d.nbmask);
 }
 
+// One job of a structure with species count T and layout L.  Shared memory:
+// [occ (occ_stride + 16), unless hbm] | search_smem_tail(T, S, nwarps) (delta
+// table, swap records, two count buffers).
 template <int T, class L>
 __device__ __noinline__ JobEnd batch_job(const SearchConst &c, const BatchStruct &d, const BatchJob &job,
                                          uint8_t *smem, unsigned long long *stats, unsigned long long *tally,
@@ -272,9 +272,11 @@ __device__ __forceinline__ JobEnd batch_dispatch_t(const SearchConst &c, const B
 // would go on with the job that stood there before.  That would explain what an
 // earlier form without it, with a plain barrier and a shared stop flag, once
 // did (other warps took the old job again); the form is not run any more, so it
-// is an explanation and not a finding.  Dynamic shared memory: occupancy of the
-// largest shared-memory structure + 16 + per-warp counts + swap records; the
-// job's constants (1.9 KB) are copied to static shared memory.
+// is an explanation and not a finding.
+//
+// Dynamic shared memory: what the largest job needs (batch_job: staged occupancy,
+// delta table, swap records, count buffers); the job's constants (SearchConst,
+// 2.1 KB) are copied to static shared memory.
 __global__ void __launch_bounds__(HEA_BATCH_THREADS, HEA_BATCH_MIN_BLOCKS)
     batch_kernel(const BatchStruct *__restrict__ structs, BatchState *states, BatchJob *jobs, BatchCtl *ctl,
                  unsigned long long *finish_ns)

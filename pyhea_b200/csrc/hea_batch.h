@@ -42,12 +42,13 @@
 // by wall time since the last finished job; on expiry the kernel sets an
 // error flag and every CTA returns.
 //
-// Occupancy in HBM (`hbm`, the default: proposals are scored from the site
-// histograms, so a search reads the occupancy only for its draws): a job copies
-// the row onto itself (reads through L2, so no stale L1 line of another SM's
-// writes is used; the copy rewrites every byte this CTA later reads) and
-// searches it through L1.  Otherwise the row is staged in the launch's shared
-// memory.
+// Proposals are scored from the site histograms, so a search reads the occupancy
+// only for its draws.  Where it lies is the host's choice (a batch stages every
+// row in shared memory when all fit, else keeps all in HBM; the server decides
+// by size).  In HBM (`hbm`) a job copies the row onto itself (reads through L2,
+// so no stale L1 line of another SM's writes is used; the copy rewrites every
+// byte this CTA later reads) and searches it through L1.  Otherwise the row is
+// staged in the launch's shared memory.
 #pragma once
 #include <cstdint>
 

@@ -1380,7 +1380,7 @@ int plan_search(hea_plan *pl, hea_stats *stats)
         stats->accepts = (int64_t)s[2];
         stats->gpu_ms = ms;
         // local-search busy time: union of the launch intervals (launches on
-        // the two streams overlap), from event times relative to ev0
+        // the survivors' stream and those of the populations ahead overlap), from event times relative to ev0
         std::vector<std::pair<float, float>> iv;
         for (int i = 0; i < pl->mc_timed; ++i) {
             float a = 0, b = 0;
@@ -1675,26 +1675,27 @@ __global__ void __launch_bounds__(256) l2_read_probe_kernel(const uint4 *buf, in
     if (acc == 0x9E3779B9u) atomicAdd(sink, 1u);
 }
 
-// Random 16-byte loads through L2 from a buffer far larger than L2, eight in
-// flight per thread: the access pattern of the site-histogram loads of
-// structures whose histograms do not fit in L2.  Indices come from the murmur3
-// finaliser of a per-thread counter, mapped to [0, n16) by a multiply-high.
+// Random 8-byte loads (a site's histogram entry) through L2 from a buffer far
+// larger than L2, eight in flight per thread: the access pattern of the
+// site-histogram loads of structures whose histograms do not fit in L2.
+// Indices come from the murmur3 finaliser of a per-thread counter: one of n16
+// 16-byte units by a multiply-high, its half by the lowest bit.
 template <bool kStream>
-__global__ void __launch_bounds__(256) dram_random_probe_kernel(const uint4 *buf, uint64_t n16, int per_thread,
+__global__ void __launch_bounds__(256) dram_random_probe_kernel(const uint2 *buf, uint64_t n16, int per_thread,
                                                                 uint32_t seed, uint32_t *sink)
 {
     uint32_t acc = 0;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     for (int i = 0; i < per_thread; i += 8) {
-        uint4 v[8];
+        uint2 v[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             const uint32_t h = fmix32(seed ^ (t * 0x9E3779B9u) ^ (uint32_t)(i + u) * 0x85EBCA6Bu);
-            const uint64_t idx = ((uint64_t)h * n16) >> 32;
+            const uint64_t idx = 2 * (((uint64_t)h * n16) >> 32) + (h & 1u);
             v[u] = kStream ? __ldcs(buf + idx) : __ldcg(buf + idx);
         }
 #pragma unroll
-        for (int u = 0; u < 8; ++u) acc ^= v[u].x ^ v[u].w;
+        for (int u = 0; u < 8; ++u) acc ^= v[u].x ^ v[u].y;
     }
     if (acc == 0x9E3779B9u) atomicAdd(sink, 1u);
 }
@@ -1728,9 +1729,9 @@ int hea_dram_random_probe(int64_t bytes, int32_t per_thread, double *out_loads_p
         for (int per_sm : {8, 32}) {
             const int grid = sms * per_sm;
             const auto kern = stream ? dram_random_probe_kernel<true> : dram_random_probe_kernel<false>;
-            kern<<<grid, 256>>>((const uint4 *)buf.p, n16, 8, 1u, (uint32_t *)sink.p);
+            kern<<<grid, 256>>>((const uint2 *)buf.p, n16, 8, 1u, (uint32_t *)sink.p);
             cudaEventRecord(e0);
-            kern<<<grid, 256>>>((const uint4 *)buf.p, n16, per_thread, 7u, (uint32_t *)sink.p);
+            kern<<<grid, 256>>>((const uint2 *)buf.p, n16, per_thread, 7u, (uint32_t *)sink.p);
             cudaEventRecord(e1);
             e = cudaEventSynchronize(e1);
             float ms = 0.0f;

@@ -7,7 +7,7 @@
 //   occ    uint8 [slots][occ_stride]   species per site, one row per slot
 //   cnt    int32 [slots][S][T][T]      pair counts that travel with their slot
 //   f2     double [slots]              squared weighted SRO error
-//   order  int32 [2P]                  slot ids: current population, then the new one
+//   order  int32 [P (W + 1)]           slot ids: survivors, then each of W new populations
 // In shared memory a slot's occupancy has the sentinel byte 0 at index N.
 #pragma once
 #include <cstdint>
@@ -588,8 +588,9 @@ __device__ __forceinline__ void delta_linear(const DeltaTab<T, S> tab, int32_t *
 //
 // Why one word: the two entries of a proposal are random loads, and what they
 // cost is set by how much of the population's histograms L2 holds and, beyond
-// it, by DRAM's random-access rate.  Measured on B200 from a 4 GiB buffer:
-// 4.8e10 random 8-byte loads/s against 2.4e10 (3.2e10 evict-first) 16-byte ones.
+// it, by DRAM's random-access rate.  Measured on B200 from a 4 GiB buffer, 32 CTAs
+// of 256 threads per SM: 4.7e10 random 8-byte loads/s (hea_dram_random_probe)
+// against 2.3e10 (3.2e10 evict-first) 16-byte ones.
 // ---------------------------------------------------------------------------
 template <int T, int S, bool kImplicit>
 struct SiteHist {
@@ -670,10 +671,9 @@ __device__ __forceinline__ uint64_t hist_species_bits(int a)
     return ((uint64_t)(a & 3) << 62) | ((uint64_t)(a >> 2) << 31);
 }
 
-// Two sites' entries, through L2.  In batches whose histograms are far larger
-// than L2 the large structures (SearchConst::hist_stream, set by the host) read
-// them evict-first, so that random lines from DRAM do not push out those that are
-// read again.
+// Two sites' entries, through L2.  Structures whose histograms are far larger
+// than L2 (SearchConst::hist_stream, set by the host) read them evict-first, so
+// that random lines from DRAM do not push out those that are read again.
 template <int W>
 __device__ __forceinline__ void load_hist_pair(const SearchConst &c, const uint64_t *hist, uint32_t s1, uint32_t s2,
                                                HistEntry<W> &p, HistEntry<W> &q)
@@ -900,7 +900,7 @@ __device__ __forceinline__ double exact_delta(const SearchConst &c, const int32_
 
 // The same by one lane alone, each of the active lanes with its own proposal.
 // Rolled loops: it is rare, and the search loop's code stays small.  Inlined, so
-// that its registers are the search loop's (as a call it cost spills there).
+// that its registers are the search loop's (as a call it cost more spills there).
 template <int T, class L, int W>
 __device__ __forceinline__ double exact_delta_lane(const SearchConst &c, const int32_t *cnt, int ab,
                                                    const HistEntry<W> &p, const HistEntry<W> &q)
@@ -938,31 +938,34 @@ __device__ __forceinline__ double exact_delta_lane(const SearchConst &c, const i
 // Few species in few shells (T S <= 6) meet that in most rounds: a plan of two
 // species in one shell (11 628 sites) took 1.79 ms a pass without the check against
 // 1.60 ms of the FP64-scored form, and is level with it (1.28 and 1.27 ms on the
-// device) with it.  More terms meet it almost never, and the check's code cost the
-// mixed batch 7 %, so they do without.  Else each candidate computes
+// device) with it.  More terms meet it almost never: compiled for all, the check
+// cost the mixed batch 7 % (56.5 -> 60.7 ms), so they do without; the line between
+// is drawn by that, not measured for each T and S.  Else each candidate computes
 // its exact D.  Returns the lane of the lowest D, lowest task on equal D, or -1
 // when no D < 0.  Convergent warp.
 template <int T, class L, int W>
 __device__ __forceinline__ int resolve(const SearchConst &c, const int32_t *cnt, bool in, bool negative, int task,
                                        int ab, const HistEntry<W> &p, const HistEntry<W> &q)
 {
-    if (T * L::S <= 6 && negative) {
-        using H = SiteHist<T, L::S, L::kImplicit>;
-        const int src = __ffs(__ballot_sync(0xFFFFFFFFu, in)) - 1;
-        const bool flip = (ab & 0xFF) > (ab >> 8);
-        const int species = flip ? (ab >> 8) | ((ab & 0xFF) << 8) : ab;
-        bool same = __shfl_sync(0xFFFFFFFFu, species, src) == species;
+    if constexpr (T * L::S <= 6) {
+        if (negative) {
+            using H = SiteHist<T, L::S, L::kImplicit>;
+            const int src = __ffs(__ballot_sync(0xFFFFFFFFu, in)) - 1;
+            const bool flip = (ab & 0xFF) > (ab >> 8);
+            const int species = flip ? (ab >> 8) | ((ab & 0xFF) << 8) : ab;
+            bool same = __shfl_sync(0xFFFFFFFFu, species, src) == species;
 #pragma unroll
-        for (int h = 0; h < H::kHalves; ++h)
+            for (int h = 0; h < H::kHalves; ++h)
 #pragma unroll
-            for (int y = 0; y < 2; ++y) {
-                const uint32_t x = q.half(h) & H::fields(h, y), z = p.half(h) & H::fields(h, y);
-                const uint32_t d = flip ? z - x : x - z;  // fields' guard bits keep differences apart
-                same = __shfl_sync(0xFFFFFFFFu, d, src) == d && same;
+                for (int y = 0; y < 2; ++y) {
+                    const uint32_t x = q.half(h) & H::fields(h, y), z = p.half(h) & H::fields(h, y);
+                    const uint32_t d = flip ? z - x : x - z;  // fields' guard bits keep differences apart
+                    same = __shfl_sync(0xFFFFFFFFu, d, src) == d && same;
+                }
+            if (__all_sync(0xFFFFFFFFu, same || !in)) {
+                const uint32_t first = __reduce_min_sync(0xFFFFFFFFu, in ? (uint32_t)task : 0xFFFFFFFFu);
+                return __ffs(__ballot_sync(0xFFFFFFFFu, in && (uint32_t)task == first)) - 1;
             }
-        if (__all_sync(0xFFFFFFFFu, same || !in)) {
-            const uint32_t first = __reduce_min_sync(0xFFFFFFFFu, in ? (uint32_t)task : 0xFFFFFFFFu);
-            return __ffs(__ballot_sync(0xFFFFFFFFu, in && (uint32_t)task == first)) - 1;
         }
     }
     uint64_t key = ~0ull;  // ~bits(D) of D < 0: more negative, smaller

@@ -13,6 +13,8 @@
 #include <chrono>
 #include <ctime>
 #include <deque>
+#include <iterator>
+#include <list>
 #include <map>
 #include <mutex>
 #include <new>
@@ -53,14 +55,25 @@ int fail(int code, const char *fmt, ...)
 // freed by one call are kept (per device and rounded size) and handed to the
 // next call that asks for the same size, so repeated searches of one shape
 // make no cudaMalloc/cudaFree (both can synchronise the device).  At most
-// kPoolCacheBytes stay cached; a failed cudaMalloc releases the cache and
-// retries.  Blocks go back to the cache only after the owning stream's work
-// has finished (every owner synchronises before freeing).
+// kPoolCacheBytes stay cached, those given back last: blocks of shapes that are
+// not searched any more make way (left in place they kept the cache full, and
+// every later batch of the mixed workload allocated and freed its buffers anew:
+// 7.0e9 to 8.1e9 evaluations/s end to end in a process that had searched other
+// plans, against 1.3e10).  A failed cudaMalloc releases the cache and retries.
+// Blocks go back to the cache only after the owning stream's work has finished
+// (every owner synchronises before freeing).
 // ---------------------------------------------------------------------------
 struct DevicePool {
+    using Key = std::pair<int, size_t>;  // device, rounded size
+    struct Block {
+        Key key;
+        void *p;
+    };
     std::mutex mu;
-    std::map<std::pair<int, size_t>, std::vector<void *>> free_;  // (device, rounded size) -> cached blocks
-    std::unordered_map<void *, std::pair<int, size_t>> live;
+    std::list<Block> blocks;  // cached, in the order they were given back
+    std::list<Block> spare;   // nodes of blocks in use, for when they come back
+    std::map<Key, std::vector<std::list<Block>::iterator>> free_;  // the same by key, in the same order
+    std::unordered_map<void *, Key> live;
     size_t cached = 0;
 };
 // never destroyed: plans may be freed during interpreter or process shutdown
@@ -85,12 +98,25 @@ void pool_release_device(DevicePool &P, int dev)
             ++it;
             continue;
         }
-        for (void *q : it->second) {
-            cudaFree(q);
+        for (auto block : it->second) {
+            cudaFree(block->p);
             P.cached -= it->first.second;
+            P.blocks.erase(block);
         }
         it = P.free_.erase(it);
     }
+}
+
+// The block given back longest ago, also the first of its key.
+void pool_release_oldest(DevicePool &P)
+{
+    const DevicePool::Block oldest = P.blocks.front();
+    P.blocks.pop_front();
+    auto it = P.free_.find(oldest.key);
+    it->second.erase(it->second.begin());
+    if (it->second.empty()) P.free_.erase(it);
+    cudaFree(oldest.p);
+    P.cached -= oldest.key.second;
 }
 
 cudaError_t dev_alloc(void **p, size_t bytes)
@@ -103,8 +129,10 @@ cudaError_t dev_alloc(void **p, size_t bytes)
     std::lock_guard<std::mutex> lk(P.mu);
     auto it = P.free_.find({dev, r});
     if (it != P.free_.end() && !it->second.empty()) {
-        *p = it->second.back();
+        const auto block = it->second.back();
+        *p = block->p;
         it->second.pop_back();
+        P.spare.splice(P.spare.end(), P.blocks, block);
         P.cached -= r;
         P.live[*p] = {dev, r};
         return cudaSuccess;
@@ -138,14 +166,20 @@ void dev_free(void *p)
         cudaFree(p);
         return;
     }
-    const std::pair<int, size_t> key = it->second;
+    const DevicePool::Key key = it->second;
     P.live.erase(it);
-    if (P.cached + key.second > kPoolCacheBytes) {
+    if (key.second > kPoolCacheBytes) {
         cudaFree(p);
         return;
     }
-    P.free_[key].push_back(p);
+    if (P.spare.empty())
+        P.blocks.emplace_back();
+    else
+        P.blocks.splice(P.blocks.end(), P.spare, P.spare.begin());
+    P.blocks.back() = DevicePool::Block{key, p};
+    P.free_[key].push_back(std::prev(P.blocks.end()));
     P.cached += key.second;
+    while (P.cached > kPoolCacheBytes) pool_release_oldest(P);
 }
 
 // ---------------------------------------------------------------------------

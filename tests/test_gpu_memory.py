@@ -92,3 +92,25 @@ def test_many_searches_leave_the_device_its_memory(form):
             k.close()
     give_back()
     assert before - free_bytes() < 64 * MIB
+
+
+def test_buffers_of_the_last_search_stay_cached():
+    """Plans of other shapes fill the block cache; a batch made after them finds its buffers there
+    when it is made again, and the cache keeps its bound."""
+    give_back()
+    start = free_bytes()
+    large = structure(L.FCC, 60, 3)  # 864 000 sites
+    for P in range(64, 73):  # about 1 GiB each, no shape twice
+        hb.Plan(large, P, 1, 64, 2, max_rounds=2).close()
+    small = structure(L.BCC, 30, 4)
+    make = lambda: hb.Batch([small], [dict(num_solutions=256, total_iter=4, parallel_task=64,  # noqa: E731
+                                           converge_depth=1, max_rounds=2)])
+    make().close()
+    kept = free_bytes()
+    assert start - kept < 9 * GIB
+    b = make()
+    assert free_bytes() == kept  # nothing allocated
+    b.close()
+    assert free_bytes() == kept
+    give_back()
+    assert start - free_bytes() < 64 * MIB

@@ -44,8 +44,8 @@
 //
 // Proposals are scored from the site histograms, so a search reads the occupancy
 // only for its draws.  Where it lies is the host's choice (a batch stages every
-// row in shared memory when all fit, else keeps all in HBM; the server decides
-// by size).  In HBM (`hbm`) a job copies the row onto itself (reads through L2,
+// row in shared memory when all fit, else keeps all in HBM; a server by its
+// hbm_sites, all in HBM unless set).  In HBM (`hbm`) a job copies the row onto itself (reads through L2,
 // so no stale L1 line of another SM's writes is used; the copy rewrites every
 // byte this CTA later reads) and searches it through L1.  Otherwise the row is
 // staged in the launch's shared memory.

@@ -1531,7 +1531,8 @@ int plan_autotune(hea_plan *pl, bool measure)
     return HEA_OK;
 }
 
-// How many new populations a search keeps in flight beside its survivors.  One
+// How many new populations a search keeps in flight beside its survivors
+// (plan_lookahead).  One
 // leaves the chip waiting for each iteration's slowest searches, merge and
 // survivors, and a population smaller than the chip never fills it; enough of
 // them keep two chips' worth of CTAs queued.  Bounded by the iterations, by

@@ -109,8 +109,8 @@ def test_buffers_of_the_last_search_stay_cached():
     kept = free_bytes()
     assert start - kept < 9 * GIB
     b = make()
-    assert free_bytes() == kept  # nothing allocated
+    assert kept - free_bytes() < 16 * MIB  # of the batch's 620 MB nothing allocated
     b.close()
-    assert free_bytes() == kept
+    assert abs(kept - free_bytes()) < 16 * MIB
     give_back()
     assert start - free_bytes() < 64 * MIB

@@ -935,12 +935,11 @@ __device__ __forceinline__ double exact_delta_lane(const SearchConst &c, const i
 // folded in).  Proposals of the same species with the same u have the same D (and
 // of swapped species with -u: the contract's terms agree bit for bit), so where
 // all candidates are such and `negative` says their D < 0, the lowest task wins.
-// Few species in few shells (T S <= 6) meet that in most rounds: a plan of two
-// species in one shell (11 628 sites) took 1.79 ms a pass without the check against
-// 1.60 ms of the FP64-scored form, and is level with it (1.28 and 1.27 ms on the
-// device) with it.  More terms meet it almost never: compiled for all, the check
-// cost the mixed batch 7 % (56.5 -> 60.7 ms), so they do without; the line between
-// is drawn by that, not measured for each T and S.  Else each candidate computes
+// Few species in few shells (T S <= 6) meet that in most rounds.  Without -> with
+// the check, BCC 18^3, 64 solutions x 384 tasks x 4 iterations: T S = 2 0.644 -> 0.629
+// ms, 3 0.592 -> 0.567, 2 x 2 0.835 -> 0.775, 4 x 1 0.608 -> 0.597; 6, 8 and 9 level.
+// More terms meet it almost never: compiled for all, its code cost the mixed batch
+// 7 % (56.5 -> 60.7 ms), so they do without.  Else each candidate computes
 // its exact D.  Returns the lane of the lowest D, lowest task on equal D, or -1
 // when no D < 0.  Convergent warp.
 template <int T, class L, int W>
